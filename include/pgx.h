@@ -99,10 +99,11 @@ enum pgx_dct_mode { PGX_DCT_RAW = 0, PGX_DCT_FWD = 1, PGX_DCT_BWD = 2, PGX_DCT_F
 /* op.k of DCT: the mode in the low bits; PGX_DCT_CTA runs an even-length transform with its
  * phases spread over the whole CTA (block barriers between FFT stages) instead of one warp per
  * line pair.  PGX_DCT_SLOT runs the FFT of a one-slot op (b <= 1) in the slot's own lines and the
- * spare slot instead of separate buffers; it needs an even tile (tb) and a length n whose n - 1 is
- * even with an FFT stage count that can be made odd (n - 1 = 2^p 3^b with p >= 2, or p = 1 and b
- * even), and refuses other lengths (NaN).  When every DCT op of a program has it, the program
- * takes no FFT buffers of shared memory. */
+ * spare slot instead of separate buffers; it needs an even tile (tb) and a length n with n - 1 even
+ * and not 2 * 3^b with odd b, and refuses other lengths (NaN).  When every DCT op of a program has
+ * it, the program takes no FFT buffers of shared memory.
+ * Transforms of even n - 1 run in 64-bit fixed point on one scale per line; a line that holds a NaN or
+ * an infinity comes out NaN throughout. */
 #define PGX_DCT_MODE_MASK 7
 #define PGX_DCT_CTA 8
 #define PGX_DCT_SLOT 16
@@ -347,11 +348,12 @@ int pgx_matrix_apply(const pgx_matrix_plan* plan, const double* in, int64_t in_s
 /* 1 if the plan is stored banded, 0 if dense. */
 int pgx_matrix_plan_is_banded(const pgx_matrix_plan* plan);
 
-/* Device tables for line programs built by the host: twiddle factors of the
- * DCT-I of n points (2(n-1) complex values exp(-2 pi i k / (2(n-1))), then the
- * n-1 doubles 0.5 + Im(tw[m]) = 1/2 - sin(pi m / (n-1)) of the folded transform),
- * and the stencil sub-diagonal table.  The returned device
- * pointer is owned by the library and valid until process exit. */
+/* Device table of DCT ops for line programs built by the host: twiddle factors of
+ * the DCT-I of n points (2(n-1) complex values exp(-2 pi i k / (2(n-1))), then the
+ * n-1 doubles 0.5 + Im(tw[m]) = 1/2 - sin(pi m / (n-1))), followed for even n-1 by
+ * the fixed-point form that the folded transform reads (csrc/pgx_fixed.cuh: 2(n-1)
+ * entries of 16 bytes and one for 1/(n-1)).  A DCT op's table has to be this one.
+ * The returned device pointer is owned by the library and valid until process exit. */
 int pgx_dct_table(int32_t n, const double** table);
 
 /* ------------------------------------------------------------ measurement

@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "pgx.h"
+#include "pgx_fixed.cuh"
 
 namespace pgx {
 int launch_single(const pgx_program* P, const pgx_instance* I, cudaStream_t s, int ntiles);
@@ -285,7 +286,9 @@ int twiddles(int n, const double** out) {
   }
   // L complex twiddles, then the fold coefficients 1/2 - sin(pi m / N) (m < N = L/2), each the
   // FP64 sum 0.5 + Im(tw[m]) that the kernels would otherwise form per point
-  std::vector<double> h(2 * (size_t)L + L / 2);
+  const int N = L / 2;
+  const bool even = (N & 1) == 0;  // the folded transform also reads fixed-point twiddles
+  std::vector<double> h(2 * (size_t)L + N + (even ? 2 * ((size_t)L + 1) : 0));
   const double pi = 3.14159265358979323846;
   for (int k = 0; k < L; ++k) {
     double a = 2.0 * pi * (double)k / (double)L;
@@ -302,6 +305,12 @@ int twiddles(int n, const double** out) {
     }
   }
   for (int m = 0; m < L / 2; ++m) h[2 * (size_t)L + m] = 0.5 + h[2 * m + 1];
+  if (even) {  // after 5N doubles (16-byte aligned): L twiddles, then 1/N
+    for (int k = 0; k <= L; ++k) {
+      const fx_tw w = k < L ? fx_twiddle(k, N) : fx_inverse(N);
+      memcpy(&h[2 * (size_t)L + N + 2 * (size_t)k], &w, sizeof w);
+    }
+  }
   double* d = nullptr;
   int rc = upload(h, &d);
   if (rc) return rc;

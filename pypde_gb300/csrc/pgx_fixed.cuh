@@ -1,0 +1,250 @@
+// 64-bit fixed-point arithmetic for the DCT-I on GB300's integer pipes.
+//
+// GB300 retires one FP64 warp instruction per ~66 cycles and SM sub-partition (measured with
+// independent DFMA / DADD / I2D chains), but a 64-bit integer add every ~2 and a 32 x 32 + 64-bit
+// multiply-add every ~4.  A transform in 64-bit integers on one scale per line therefore issues
+// about a fifth of the cycles of the same transform in FP64 -- and it is more accurate: every point
+// carries about 58 bits below the line's absolute sum, where FP64 carries 53 below each partial sum.
+//
+// Numbers.  A line is scaled by 2^k so that the sum of its absolute values is below 2^58; every
+// intermediate of the transform (partial DFT sums of two lines and the sums of their parts, the cosine
+// sum, the scan) then stays below 2^61, so no stage needs a range check.  Coefficients (cosines, 1/N) are integers over 2^62,
+// held as a high and a balanced low word, W 2^62 = wh 2^32 + wl, |W| <= 1 (1 itself included).
+// A product drops only the low x low word product (below one unit, of either sign) and rounds the
+// cross terms, so it is within about one unit (2^-58 of the line's absolute sum) and has no bias.
+//
+// Host and device code give the same integers (plain C++ operations only).
+#ifndef PGX_FIXED_CUH
+#define PGX_FIXED_CUH
+
+#include <stdint.h>
+
+#ifdef __CUDACC__
+#define PGX_HD __host__ __device__ __forceinline__
+#else
+#define PGX_HD inline
+#endif
+
+#if defined(__CUDA_ARCH__)
+PGX_HD uint64_t fx_bits(double x) { return (uint64_t)__double_as_longlong(x); }
+PGX_HD double fx_double(uint64_t b) { return __longlong_as_double((long long)b); }
+PGX_HD int fx_clz(uint64_t a) { return __clzll((long long)a); }
+PGX_HD uint64_t fx_mulhi(uint64_t a, uint64_t b) { return __umul64hi(a, b); }
+PGX_HD int64_t fx_mad(int32_t a, int32_t b, int64_t c) {
+  int64_t d;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+  return d;
+}
+#else
+#include <string.h>
+PGX_HD uint64_t fx_bits(double x) {
+  uint64_t b;
+  memcpy(&b, &x, sizeof b);
+  return b;
+}
+PGX_HD double fx_double(uint64_t b) {
+  double x;
+  memcpy(&x, &b, sizeof x);
+  return x;
+}
+PGX_HD int fx_clz(uint64_t a) { return a ? __builtin_clzll(a) : 64; }
+PGX_HD uint64_t fx_mulhi(uint64_t a, uint64_t b) { return (uint64_t)(((unsigned __int128)a * b) >> 64); }
+// two's complement wrap-around, as the device's multiply-add
+PGX_HD int64_t fx_mad(int32_t a, int32_t b, int64_t c) {
+  return (int64_t)((uint64_t)((int64_t)a * b) + (uint64_t)c);
+}
+#endif
+
+// ---------------------------------------------------------------- products
+struct fx_cut_t {
+  int32_t h, l;  // x = h 2^32 + l, l in [-2^31, 2^31)
+};
+PGX_HD fx_cut_t fx_cut(int64_t x) {
+  fx_cut_t s;
+  s.l = (int32_t)(uint32_t)(uint64_t)x;
+  s.h = (int32_t)(x >> 32) + (int32_t)((uint32_t)s.l >> 31);
+  return s;
+}
+struct fx_w {
+  int32_t h, l;  // W = (h 2^32 + l) / 2^62, l balanced
+};
+PGX_HD fx_w fx_coef(int64_t w62) {
+  const fx_cut_t s = fx_cut(w62);
+  fx_w w;
+  w.h = s.h;
+  w.l = s.l;
+  return w;
+}
+// x W for |x| < 2^61, |W| <= 1:  (xh wh 2^64 + (xh wl + xl wh) 2^32) / 2^62
+PGX_HD int64_t fx_mul(int64_t x, fx_w w) {
+  const fx_cut_t s = fx_cut(x);
+  const int64_t t = fx_mad(s.h, w.l, fx_mad(s.l, w.h, (int64_t)1 << 29));
+  return fx_mad((int32_t)((uint32_t)s.h << 2), w.h, t >> 30);
+}
+
+struct fx2 {
+  int64_t x, y;
+};
+struct fx_tw {  // one table entry: cos and -sin of an angle, 16 bytes
+  int32_t rh, rl, ih, il;
+};
+PGX_HD fx2 fx_add(fx2 a, fx2 b) {
+  fx2 r;
+  r.x = a.x + b.x;
+  r.y = a.y + b.y;
+  return r;
+}
+PGX_HD fx2 fx_sub(fx2 a, fx2 b) {
+  fx2 r;
+  r.x = a.x - b.x;
+  r.y = a.y - b.y;
+  return r;
+}
+PGX_HD fx2 fx_mi(fx2 a, fx2 b) {  // a - i b
+  fx2 r;
+  r.x = a.x + b.y;
+  r.y = a.y - b.x;
+  return r;
+}
+PGX_HD fx2 fx_pi(fx2 a, fx2 b) {  // a + i b
+  fx2 r;
+  r.x = a.x - b.y;
+  r.y = a.y + b.x;
+  return r;
+}
+// v (cos + i (-sin)); the cross terms of both products of a component share one shift
+PGX_HD fx2 fx_cmul(fx2 v, fx_tw w) {
+  const fx_cut_t a = fx_cut(v.x), b = fx_cut(v.y);
+  const int32_t a4 = (int32_t)((uint32_t)a.h << 2), b4 = (int32_t)((uint32_t)b.h << 2);
+  const int32_t nh = -w.ih, nl = (int32_t)(0u - (uint32_t)w.il);
+  const int64_t half = (int64_t)1 << 29;
+  const int64_t tr = fx_mad(b.h, nl, fx_mad(b.l, nh, fx_mad(a.h, w.rl, fx_mad(a.l, w.rh, half))));
+  const int64_t ti = fx_mad(b.h, w.rl, fx_mad(b.l, w.rh, fx_mad(a.h, w.il, fx_mad(a.l, w.ih, half))));
+  fx2 r;
+  r.x = fx_mad(a4, w.rh, fx_mad(b4, nh, tr >> 30));
+  r.y = fx_mad(a4, w.ih, fx_mad(b4, w.rh, ti >> 30));
+  return r;
+}
+
+// ------------------------------------------------------- doubles in and out
+// Scale of a line: kx = 1027 + q when the sum of its absolute values is below 2^q; a point becomes
+// round(x 2^(58 - q)) and an integer v stands for v 2^(kx - 1085).
+// kx is at least FX_KX_MIN: a line of subnormal numbers needs no finer unit than that scale's.
+// FX_BAD: a NaN or an infinity in the line; FX_ZERO: nothing but zeros.
+enum { FX_KX0 = 1027, FX_P0 = 1085, FX_KX_MIN = 6, FX_BAD = 1 << 20, FX_ZERO = 1 << 21 };
+
+// x 2^(FX_P0 - kx) (times 2 with dbl, negated with neg) rounded to nearest, halves away from zero
+PGX_HD int64_t fx_from_double(double x, int kx, int neg, int dbl) {
+  const uint64_t b = fx_bits(x);
+  const uint32_t hi = (uint32_t)(b >> 32);
+  int e = (int)((hi >> 20) & 0x7ff);
+  uint32_t mh = hi & 0xfffff;
+  if (e) mh |= 0x100000;
+  else e = 1;
+  int s = kx - 1 - e - dbl;  // one bit more than wanted, for the rounding
+  s = s < 0 ? 0 : (s > 63 ? 63 : s);
+  const uint64_t m = (((uint64_t)mh << 32) | (uint32_t)b) << 10;
+  const int64_t y = (int64_t)(((m >> s) + 1) >> 1);
+  const int64_t sg = -(int64_t)((hi >> 31) ^ (uint32_t)neg);
+  return (y ^ sg) - sg;
+}
+
+// v 2^p rounded to nearest (halves away from zero); overflow gives infinity, small results subnormals
+PGX_HD double fx_to_double(int64_t v, int p) {
+  const uint64_t sg = (uint64_t)(v >> 63);
+  uint64_t a = ((uint64_t)v ^ sg) - sg;
+  if (a == 0) return 0.0;
+  const int lz = fx_clz(a);
+  a <<= lz;
+  const int e = 1086 + p - lz;  // biased exponent of a 2^(p - lz), a in [2^63, 2^64)
+  uint64_t r;
+  if (e >= 1 && e <= 2046) {
+    r = (a >> 11) + ((a >> 10) & 1) + ((uint64_t)(e - 1) << 52);  // a carry moves into the exponent
+  } else if (e > 2046) {
+    r = 0x7FF0000000000000ULL;
+  } else {
+    const int sh = 11 - e;  // 10 + (1 - e)
+    r = sh > 63 ? 0 : ((a >> sh) + 1) >> 1;
+  }
+  return fx_double(r | (sg & 0x8000000000000000ULL));
+}
+
+// Exponent q with f 2^r < 2^q for a positive normal float f (a little above its sum's rounding)
+PGX_HD int fx_exponent(float f, int r) {
+  uint32_t u;
+#if defined(__CUDA_ARCH__)
+  u = __float_as_uint(f * 1.0001f);
+#else
+  const float g = f * 1.0001f;
+  memcpy(&u, &g, sizeof u);
+#endif
+  return (int)((u >> 23) & 0xff) - 126 + r;
+}
+
+// ------------------------------------------------------------ cosine tables
+// cos and sin of 2 pi k / L (0 <= k < L, L a multiple of 4 below 2^13) times 2^62, within about a
+// unit: the angle is reduced to an eighth of a turn in integers, then summed as a Taylor series in
+// 64-bit fractions.
+PGX_HD void fx_cos_sin(int k, int L, int64_t* c62, int64_t* s62) {
+  const int64_t k8 = 8 * (int64_t)k;
+  const int oct = (int)(k8 / L);
+  int64_t rem = k8 - (int64_t)oct * L;           // angle = (oct + rem / L) pi / 4
+  if (oct & 1) rem = L - rem;                    // measured from the nearest multiple of pi / 2
+  uint64_t f = 0;                                // rem / L as a 64-bit fraction (rem == L: below)
+  uint64_t r = (uint64_t)rem;
+  int64_t c, s;
+  if (rem == L) {  // exactly pi / 4: sqrt(1/2) 2^62, rounded
+    c = s = 3260954456333195553LL;
+  } else {
+    for (int i = 0; i < 4; ++i) {
+      r <<= 16;
+      f = (f << 16) | (r / (uint64_t)L);
+      r %= (uint64_t)L;
+    }
+    const uint64_t kQuarterPi = 0xC90FDAA22168C235ULL;  // pi / 4 as a 64-bit fraction, rounded
+    const uint64_t t = fx_mulhi(f, kQuarterPi);         // the angle, radians, 64-bit fraction
+    const uint64_t t2 = fx_mulhi(t, t);
+    // Horner: cos = 1 - t2/2 (1 - t2/12 (1 - ...)), sin = t (1 - t2/6 (1 - t2/20 (...)))
+    uint64_t cs = ~0ULL, sn = ~0ULL;  // 1 to the last place
+    for (int j = 22; j >= 4; j -= 2) cs = ~0ULL - fx_mulhi(t2, cs) / (uint64_t)(j * (j - 1));
+    for (int j = 21; j >= 3; j -= 2) sn = ~0ULL - fx_mulhi(t2, sn) / (uint64_t)(j * (j - 1));
+    const uint64_t half = fx_mulhi(t2, cs) >> 1;        // 1 - cos
+    c = ((int64_t)1 << 62) - (int64_t)((half + 2) >> 2);
+    s = (int64_t)((fx_mulhi(t, sn) + 2) >> 2);
+  }
+  int64_t cq = c, sq = s;  // within the quarter turn: the angle of octants 1, 3, ... counts backwards
+  if (oct & 1) {
+    cq = s;
+    sq = c;
+  }
+  switch (oct >> 1) {
+    case 0: *c62 = cq; *s62 = sq; break;
+    case 1: *c62 = -sq; *s62 = cq; break;
+    case 2: *c62 = -cq; *s62 = -sq; break;
+    default: *c62 = sq; *s62 = -cq; break;
+  }
+}
+// table entry k of a length-N transform (N even): exp(-2 pi i k / (2N))
+PGX_HD fx_tw fx_twiddle(int k, int N) {
+  int64_t c, s;
+  fx_cos_sin(k, 2 * N, &c, &s);
+  const fx_w a = fx_coef(c), b = fx_coef(-s);
+  fx_tw w;
+  w.rh = a.h; w.rl = a.l; w.ih = b.h; w.il = b.l;
+  return w;
+}
+// 1 / N = c / 2^62 * 2^-g with c in (2^61, 2^62]; the entry after the 2N twiddles: (ch, cl, g, 0)
+PGX_HD fx_tw fx_inverse(int N) {
+  int g = 0;
+  while ((2 << g) <= N) ++g;
+  const uint64_t one = (uint64_t)1 << 62;
+  const uint64_t q = one / (uint64_t)N, r = one % (uint64_t)N;
+  const int64_t c = (int64_t)((q << g) + ((r << g) + (uint64_t)N / 2) / (uint64_t)N);
+  const fx_w a = fx_coef(c);
+  fx_tw w;
+  w.rh = a.h; w.rl = a.l; w.ih = g; w.il = 0;
+  return w;
+}
+
+#undef PGX_HD
+#endif  // PGX_FIXED_CUH

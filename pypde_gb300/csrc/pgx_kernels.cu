@@ -24,6 +24,7 @@
 
 #include "pgx.h"
 #include "pgx_exact.cuh"
+#include "pgx_fixed.cuh"
 
 // Complex elements per line pair in each FFT buffer for DCT lengths up to n:
 // n - 1 for the folded algorithm (even n - 1), 2(n - 1) for paired lines.
@@ -67,6 +68,38 @@ __host__ __device__ inline bool pgx_fft_in_slot(const pgx_program& P) {
   return any && !(P.tb & 1);
 }
 
+// Slots that have to start as zeros: those whose first op is not one that writes the whole line, tail
+// included (LOAD; COPY into it).  The spare (bit nslots) is written whole by every op that leaves
+// data in it.  The fused passes load every slot first, so their tiles clear nothing.
+inline unsigned pgx_init_mask(const pgx_program& P) {
+  unsigned seen = 0, need = 0;
+  auto touch = [&](int slot, bool whole) {
+    const unsigned b = 1u << slot;
+    if (!(seen & b) && !whole) need |= b;
+    seen |= b;
+  };
+  for (int o = 0; o < P.nops; ++o) {
+    const pgx_op& op = P.ops[o];
+    switch (op.code) {
+      case PGX_OP_LOAD: touch(op.a, true); break;
+      case PGX_OP_COPY:
+        touch(op.b, false);
+        touch(op.a, true);
+        break;
+      case PGX_OP_AXPY:
+      case PGX_OP_MUL:
+        touch(op.b, false);
+        touch(op.a, false);
+        break;
+      case PGX_OP_DIFF: case PGX_OP_DIFF_T: case PGX_OP_TDMA2: case PGX_OP_FDMA: case PGX_OP_FDMA_T: case PGX_OP_DCT:
+        for (int k = 0; k < (op.b > 1 ? op.b : 1); ++k) touch(op.a + k, false);
+        break;
+      default: touch(op.a, false); break;
+    }
+  }
+  return need;
+}
+
 namespace pgx {
 
 // 2k for k < PGX_LMAX: multipliers of the derivative recurrence, read through
@@ -81,11 +114,36 @@ constexpr TwoK make_twok() {
 }
 __constant__ TwoK c_twok = make_twok();
 
+// x / d by a multiply-high for x < 2^18, d < 2^12 (offsets into a tile are below 2^15, lines and
+// chunks below 2^12): m = ceil(2^32 / d), exact while x (m d - 2^32) < 2^32.  A runtime division
+// is ~20 instructions, and every element of the load, store and stencil loops and every butterfly
+// needs one or two.
+struct DivTable {
+  uint32_t m[PGX_LMAX + 16];
+};
+constexpr DivTable make_divs() {
+  DivTable t{};
+  for (uint32_t d = 1; d < PGX_LMAX + 16; ++d) t.m[d] = 0xffffffffu / d + 1u;
+  return t;
+}
+__constant__ DivTable c_divs = make_divs();
+struct FastDiv {  // 1 <= d < PGX_LMAX + 16
+  uint32_t d, m;
+  __device__ __forceinline__ explicit FastDiv(int d_) : d((uint32_t)d_), m(c_divs.m[d_]) {}
+  __device__ __forceinline__ int div(int x) const { return d == 1 ? x : (int)__umulhi((uint32_t)x, m); }
+};
+
+// The CTA's dynamic shared memory.  Everything in it is named by its offset in doubles, and the
+// pointers are formed from this array where they are used, so that the compiler sees shared-memory
+// accesses with 32-bit addresses (through a stored pointer each access is a generic one with 64-bit
+// address arithmetic, about as many instructions again as the work).
+extern __shared__ __align__(16) double smem_dyn[];
+
 struct Ctx {
-  double* sm;       // slot buffers
-  double2* f0;      // FFT ping buffer
-  double2* f1;      // FFT pong buffer
-  double* ybuf;     // one scalar per line (DCT-I: y_1 of the folded algorithm)
+  int sm;           // slot buffers
+  int f0;           // FFT ping buffer
+  int f1;           // FFT pong buffer
+  int ybuf;         // one scalar per line (DCT-I: the line's scale)
   int tb, lcap, nthreads, tid;
   int fft_stride;   // complex elements per pair in the FFT buffers
   int l0, nlines;   // first line of the tile, lines of the instance
@@ -95,14 +153,10 @@ struct Ctx {
 };
 
 __device__ __forceinline__ double* slot_ptr(const Ctx& c, int s) {
-  return c.sm + (size_t)c.phys[s] * c.tb * c.lcap;
-}
-// Slot s0 + sl of a multi-slot op whose slot s0 is x0: sl == 0 (every one-slot op) reads no slot map.
-__device__ __forceinline__ double* op_slot(const Ctx& c, double* x0, int s0, int sl) {
-  return sl == 0 ? x0 : slot_ptr(c, s0 + sl);
+  return smem_dyn + (c.sm + c.phys[s] * c.tb * c.lcap);
 }
 __device__ __forceinline__ double* spare_ptr(const Ctx& c) {
-  return c.sm + (size_t)c.spare * c.tb * c.lcap;
+  return smem_dyn + (c.sm + c.spare * c.tb * c.lcap);
 }
 __device__ __forceinline__ void swap_spare(Ctx& c, int s) {
   int t = c.phys[s];
@@ -111,8 +165,14 @@ __device__ __forceinline__ void swap_spare(Ctx& c, int s) {
 }
 
 __device__ __forceinline__ double op_alpha(const pgx_op& op, const pgx_instance& I) {
-  return op.par >= 0 ? op.alpha * I.par[op.par] : op.alpha;
+  if (op.par < 0) return op.alpha;
+  const double p = I.par[op.par];
+  return __double_as_longlong(op.alpha) == 0x3ff0000000000000LL ? p : op.alpha * p;
 }
+
+// Whether alpha is 1, on its bits: a floating-point compare takes the FP64 pipe (66 cycles a warp),
+// and inside an element loop it was a third of a LOAD's and a STORE's time.
+__device__ __forceinline__ bool is_one(double alpha) { return __double_as_longlong(alpha) == 0x3ff0000000000000LL; }
 
 // Geometry of array `a` seen from a pass along `axis`.
 struct View {
@@ -139,144 +199,129 @@ __device__ void zero_tail(const Ctx& c, double* b, int from) {
   const int c_tid = c.tid;
   int w = c_lcap - from;
   if (w <= 0) return;
+  const FastDiv fw(w);
   for (int idx = c_tid; idx < c_tb * w; idx += c_nthreads) {
-    int t = idx / w, i = from + idx % w;
-    b[t * c_lcap + i] = 0.0;
+    const int t = fw.div(idx);
+    b[t * c_lcap + from + idx - t * w] = 0.0;
   }
 }
 
 // ------------------------------------------------------------------ load/store
+// The element loops of LOAD and STORE, one build each for alpha == 1 (ONE): a multiply by it, or a
+// predicated-off one, costs as much as all the rest of an element (66 cycles a warp).
 // mode 0: slot = alpha*arr (length n, zero beyond the array), 1: +=, 2: *=
-template <int KU>
-__device__ void op_load(Ctx& c, const pgx_op& op, const pgx_instance& I, int axis, int mode) {
+template <int KU, bool ONE, int MODE>
+__device__ __forceinline__ void load_loop(const Ctx& c, const View& v, double* s, int n, double alpha) {
   const int c_tb = c.tb;
   const int c_lcap = c.lcap;
   const int c_nthreads = c.nthreads;
-  const int c_tid = c.tid;
-  const int c_l0 = c.l0;
-  const int c_nlines = c.nlines;
-  const View v = view_of(I.arr[op.arr], axis);
-  const double alpha = op_alpha(op, I);
-  int n;
-  if (mode == 0) {
-    n = I.len[op.len];
-    c.slen[op.a] = n;
-  } else {
-    n = c.slen[op.a];
-  }
-  double* s = slot_ptr(c, op.a);
-  const int tb = c_tb;
+  const int l0 = c.l0;
+  const int nl = min(v.nl, c.nlines);
   const bool contig = (v.se == 1);
-  const int total = tb * n;
-  // up to kU elements a thread per round, all their global loads issued before the first store to
-  // the slot: the stores go through generic pointers, which the compiler may not move loads across,
-  // so one element at a time would wait out a full memory latency per element (the build for
+  const int total = c_tb * n;
+  const FastDiv fd(contig ? max(n, 1) : c_tb);
+  // up to KU elements a thread per round, all their global loads issued before the first store to
+  // the slot, so a round waits out one memory latency, not one an element (the build for
   // launches of fewer CTAs than SMs, KU = 1, keeps the shorter single-element loop)
-  constexpr int kU = KU;
-  if (total <= c_nthreads) {  // at most one element a thread (single instances, short lines)
-    if (c_tid < total) {
-      int t, i;
-      if (contig) { t = c_tid / n; i = c_tid - t * n; }
-      else { i = c_tid / tb; t = c_tid - i * tb; }
-      const int line = c_l0 + t;
-      double x = 0.0;
-      if (i < v.ne && line < v.nl && line < c_nlines) x = v.p[(int64_t)i * v.se + (int64_t)line * v.sl];
-      double* d = s + t * c_lcap + i;
-      if (mode == 0) *d = alpha == 1.0 ? x : alpha * x;
-      else if (mode == 1) *d = fma(alpha, x, *d);
-      else *d = (alpha == 1.0 ? x : alpha * x) * (*d);
-    }
-    if (mode == 0) zero_tail(c, s, n);
-    return;
-  }
-  for (int base = c_tid; base < total; base += kU * c_nthreads) {
-    double x[kU];
-    int off[kU];
+  for (int base = c.tid; base < total; base += KU * c_nthreads) {
+    double x[KU];
+    int off[KU];
 #pragma unroll
-    for (int u = 0; u < kU; ++u) {
+    for (int u = 0; u < KU; ++u) {
       const int idx = base + u * c_nthreads;
       x[u] = 0.0;
       off[u] = -1;
       if (idx < total) {
         int t, i;
-        if (contig) { t = idx / n; i = idx - t * n; }
-        else { i = idx / tb; t = idx - i * tb; }
-        const int line = c_l0 + t;
+        if (contig) { t = fd.div(idx); i = idx - t * n; }
+        else { i = fd.div(idx); t = idx - i * c_tb; }
+        const int line = l0 + t;
         off[u] = t * c_lcap + i;
-        if (i < v.ne && line < v.nl && line < c_nlines) x[u] = v.p[(int64_t)i * v.se + (int64_t)line * v.sl];
+        if (i < v.ne && line < nl) x[u] = v.p[(int64_t)i * v.se + (int64_t)line * v.sl];
       }
     }
 #pragma unroll
-    for (int u = 0; u < kU; ++u) {
+    for (int u = 0; u < KU; ++u) {
       if (off[u] < 0) continue;
       double* d = s + off[u];
-      if (mode == 0) *d = alpha == 1.0 ? x[u] : alpha * x[u];
-      else if (mode == 1) *d = fma(alpha, x[u], *d);
-      else *d = (alpha == 1.0 ? x[u] : alpha * x[u]) * (*d);
+      if (MODE == 0) *d = ONE ? x[u] : alpha * x[u];
+      else if (MODE == 1) *d = ONE ? x[u] + *d : fma(alpha, x[u], *d);
+      else *d = (ONE ? x[u] : alpha * x[u]) * (*d);
     }
   }
-  if (mode == 0) zero_tail(c, s, n);  // [n, lcap) of every line: no element the loop writes
+}
+template <int KU>
+__device__ void op_load(Ctx& c, const pgx_op& op, const pgx_instance& I, int axis, int mode) {
+  const View v = view_of(I.arr[op.arr], axis);
+  const double alpha = op_alpha(op, I);
+  const bool one = is_one(alpha);
+  if (mode == 0) c.slen[op.a] = I.len[op.len];
+  const int n = c.slen[op.a];
+  double* s = slot_ptr(c, op.a);
+  if (mode == 0) {
+    if (one) load_loop<KU, true, 0>(c, v, s, n, alpha);
+    else load_loop<KU, false, 0>(c, v, s, n, alpha);
+    zero_tail(c, s, n);  // [n, lcap) of every line: no element the loop writes
+  } else if (mode == 1) {
+    if (one) load_loop<KU, true, 1>(c, v, s, n, alpha);
+    else load_loop<KU, false, 1>(c, v, s, n, alpha);
+  } else {
+    load_loop<KU, false, 2>(c, v, s, n, alpha);
+  }
 }
 
-template <int KU>
-__device__ void op_store(const Ctx& c, const pgx_op& op, const pgx_instance& I, int axis, bool add) {
+template <int KU, bool ONE, bool ADD>
+__device__ __forceinline__ void store_loop(const Ctx& c, const View& v, const double* s, double alpha) {
   const int c_tb = c.tb;
   const int c_lcap = c.lcap;
   const int c_nthreads = c.nthreads;
-  const int c_tid = c.tid;
-  const int c_l0 = c.l0;
-  const int c_nlines = c.nlines;
-  const View v = view_of(I.arr[op.arr], axis);
-  const double alpha = op_alpha(op, I);
-  const double* s = slot_ptr(c, op.a);
+  const int l0 = c.l0;
+  const int nl = min(v.nl, c.nlines);
   const int n = v.ne;
-  const int tb = c_tb;
   const bool contig = (v.se == 1);
-  const int total = tb * n;
-  // up to kU elements a thread per round, every load (the slot's and, to accumulate, the array's)
+  const int total = c_tb * n;
+  const FastDiv fd(contig ? max(n, 1) : c_tb);
+  // up to KU elements a thread per round, every load (the slot's and, to accumulate, the array's)
   // before the first store: one memory latency per round, not per element
-  constexpr int kU = KU;
-  if (total <= c_nthreads) {  // at most one element a thread (single instances, short lines)
-    if (c_tid < total) {
-      int t, i;
-      if (contig) { t = c_tid / n; i = c_tid - t * n; }
-      else { i = c_tid / tb; t = c_tid - i * tb; }
-      const int line = c_l0 + t;
-      if (line < v.nl && line < c_nlines) {
-        const double x = s[t * c_lcap + i];
-        double* d = v.p + (int64_t)i * v.se + (int64_t)line * v.sl;
-        if (add) *d = fma(alpha, x, *d);
-        else *d = alpha == 1.0 ? x : alpha * x;
-      }
-    }
-    return;
-  }
-  for (int base = c_tid; base < total; base += kU * c_nthreads) {
-    double x[kU], old[kU];
-    double* dp[kU];
+  for (int base = c.tid; base < total; base += KU * c_nthreads) {
+    double x[KU], old[KU];
+    double* dp[KU];
 #pragma unroll
-    for (int u = 0; u < kU; ++u) {
+    for (int u = 0; u < KU; ++u) {
       const int idx = base + u * c_nthreads;
       dp[u] = nullptr;
       x[u] = old[u] = 0.0;
       if (idx < total) {
         int t, i;
-        if (contig) { t = idx / n; i = idx - t * n; }
-        else { i = idx / tb; t = idx - i * tb; }
-        const int line = c_l0 + t;
-        if (line < v.nl && line < c_nlines) {
+        if (contig) { t = fd.div(idx); i = idx - t * n; }
+        else { i = fd.div(idx); t = idx - i * c_tb; }
+        const int line = l0 + t;
+        if (line < nl) {
           x[u] = s[t * c_lcap + i];
           dp[u] = v.p + (int64_t)i * v.se + (int64_t)line * v.sl;
-          if (add) old[u] = *dp[u];
+          if (ADD) old[u] = *dp[u];
         }
       }
     }
 #pragma unroll
-    for (int u = 0; u < kU; ++u) {
+    for (int u = 0; u < KU; ++u) {
       if (!dp[u]) continue;
-      if (add) *dp[u] = fma(alpha, x[u], old[u]);
-      else *dp[u] = alpha == 1.0 ? x[u] : alpha * x[u];
+      if (ADD) *dp[u] = ONE ? x[u] + old[u] : fma(alpha, x[u], old[u]);
+      else *dp[u] = ONE ? x[u] : alpha * x[u];
     }
+  }
+}
+template <int KU>
+__device__ void op_store(const Ctx& c, const pgx_op& op, const pgx_instance& I, int axis, bool add) {
+  const View v = view_of(I.arr[op.arr], axis);
+  const double alpha = op_alpha(op, I);
+  const double* s = slot_ptr(c, op.a);
+  if (is_one(alpha)) {
+    if (add) store_loop<KU, true, true>(c, v, s, alpha);
+    else store_loop<KU, true, false>(c, v, s, alpha);
+  } else {
+    if (add) store_loop<KU, false, true>(c, v, s, alpha);
+    else store_loop<KU, false, false>(c, v, s, alpha);
   }
 }
 
@@ -287,6 +332,7 @@ __device__ void op_pointwise(Ctx& c, const pgx_op& op, const pgx_instance& I) {
   const int c_nthreads = c.nthreads;
   const int c_tid = c.tid;
   const double alpha = op_alpha(op, I);
+  const bool one = is_one(alpha);
   double* a = slot_ptr(c, op.a);
   const double* b = op.b >= 0 ? slot_ptr(c, op.b) : nullptr;
   int n = c.slen[op.a];
@@ -296,16 +342,22 @@ __device__ void op_pointwise(Ctx& c, const pgx_op& op, const pgx_instance& I) {
     else if (nb > n) n = nb;
     c.slen[op.a] = n;
   }
+  const FastDiv fn(n > 0 ? n : 1);
   for (int idx = c_tid; idx < c_tb * n; idx += c_nthreads) {
-    int t = idx / n, i = idx - t * n;
-    int o = t * c_lcap + i;
+    const int t = fn.div(idx);
+    const int o = t * c_lcap + idx - t * n;
     switch (op.code) {
       case PGX_OP_SCALE: a[o] *= alpha; break;
       case PGX_OP_AXPY: a[o] = fma(alpha, b[o], a[o]); break;
-      case PGX_OP_MUL: a[o] = (alpha == 1.0 ? b[o] : alpha * b[o]) * a[o]; break;
-      case PGX_OP_COPY: a[o] = alpha == 1.0 ? b[o] : alpha * b[o]; break;
+      case PGX_OP_MUL: a[o] *= b[o]; break;
+      default: a[o] = b[o]; break;
     }
   }
+  if (!one && (op.code == PGX_OP_MUL || op.code == PGX_OP_COPY))
+    for (int idx = c_tid; idx < c_tb * n; idx += c_nthreads) {  // the same elements as above
+      const int t = fn.div(idx);
+      a[t * c_lcap + idx - t * n] *= alpha;
+    }
   if (op.code == PGX_OP_COPY) zero_tail(c, a, n);  // [n, lcap): no element the loop reads or writes
 }
 
@@ -329,6 +381,7 @@ __device__ void op_stencil(Ctx& c, const pgx_op& op, const pgx_instance& I) {
   double* y = spare_ptr(c);
   const int M = c.slen[op.a], N = M + 2;
   const int total = c_tb * c_lcap;
+  const FastDiv fl(c_lcap);
   constexpr int kU = KU;  // the table loads of kU elements before their stores
   for (int base = c_tid; base < total; base += kU * c_nthreads) {
     double r[kU];
@@ -337,7 +390,7 @@ __device__ void op_stencil(Ctx& c, const pgx_op& op, const pgx_instance& I) {
       const int idx = base + u * c_nthreads;
       r[u] = 0.0;
       if (idx < total) {
-        const int t = idx / c_lcap, i = idx - t * c_lcap;
+        const int t = fl.div(idx), i = idx - t * c_lcap;
         if (i < N) {
           const double* xl = x + t * c_lcap;
           r[u] = i < M ? xl[i] : 0.0;
@@ -365,6 +418,7 @@ __device__ void op_stencil_t(Ctx& c, const pgx_op& op, const pgx_instance& I) {
   double* y = spare_ptr(c);
   const int N = c.slen[op.a], M = N - 2;
   const int total = c_tb * c_lcap;
+  const FastDiv fl(c_lcap);
   constexpr int kU = KU;  // the table loads of kU elements before their stores
   for (int base = c_tid; base < total; base += kU * c_nthreads) {
     double r[kU];
@@ -373,7 +427,7 @@ __device__ void op_stencil_t(Ctx& c, const pgx_op& op, const pgx_instance& I) {
       const int idx = base + u * c_nthreads;
       r[u] = 0.0;
       if (idx < total) {
-        const int t = idx / c_lcap, i = idx - t * c_lcap;
+        const int t = fl.div(idx), i = idx - t * c_lcap;
         if (i < M) {
           const double* xl = x + t * c_lcap;
           r[u] = fma(__ldg(sd + i), xl[i + 2], xl[i]);
@@ -818,6 +872,7 @@ __device__ void op_banded(Ctx& c, const pgx_op& op, const pgx_instance& I) {
   const double* x = slot_ptr(c, op.a);
   double* y = spare_ptr(c);
   const int total = c_tb * c_lcap;
+  const FastDiv fl(c_lcap);
   constexpr int kU = KU > 2 ? 2 : KU;  // the matrix loads of kU rows before their stores
   for (int base = c_tid; base < total; base += kU * c_nthreads) {
     double acc[kU];
@@ -826,7 +881,7 @@ __device__ void op_banded(Ctx& c, const pgx_op& op, const pgx_instance& I) {
       const int idx = base + u * c_nthreads;
       acc[u] = 0.0;
       if (idx < total) {
-        const int t = idx / c_lcap, r = idx - t * c_lcap;
+        const int t = fl.div(idx), r = idx - t * c_lcap;
         if (r < rows) {
           const double* xl = x + t * c_lcap;
           for (int d = 0; d < nd; ++d) {
@@ -913,8 +968,9 @@ __device__ void op_dense(Ctx& c, const pgx_op& op, const pgx_instance& I) {
   const double* x = slot_ptr(c, op.a);
   double* y = spare_ptr(c);
   zero_tail(c, y, rows);
+  const FastDiv ft(c_tb);
   for (int idx = c_tid; idx < c_tb * rows; idx += c_nthreads) {
-    int r = idx / c_tb, t = idx - r * c_tb;
+    const int r = ft.div(idx), t = idx - r * c_tb;
     const double* xl = x + t * c_lcap;
     const double* Ar = A + (size_t)r * cols;
     double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
@@ -1123,492 +1179,645 @@ __device__ __forceinline__ void stage_dispatch(int R, const Ctx& c, const double
   else stockham_stage<3, FIRST, LAST>(c, src, dst, tw, L, Ns, npairs, x, ds, tws);
 }
 
-// Radix plan of the length-N FFT: every factor 3 first (the first stage has no twiddles, and a
-// twiddled radix-3 stage costs the most FP64 instructions per point), then 4s, then one 2.
-struct RadixPlan {
-  int n3, n4, n2;  // stages of radix 3, then 4, then 2
-  __device__ __forceinline__ int stages() const { return n3 + n4 + n2; }
-  __device__ __forceinline__ int at(int s) const { return s < n3 ? 3 : (s < n3 + n4 ? 4 : 2); }
-};
-__device__ __forceinline__ RadixPlan radix_plan(int N, int& rest, bool radix2 = false) {
-  RadixPlan p{0, 0, 0};
-  int m = N;
-  while (m % 3 == 0) { ++p.n3; m /= 3; }
-  if (radix2) {
-    while (m % 2 == 0) { ++p.n2; m /= 2; }
-  } else {
-    while (m % 4 == 0) { ++p.n4; m /= 4; }
-    if (m % 2 == 0) { ++p.n2; m /= 2; }
-  }
-  rest = m;  // 1 for every length with a twiddle table (n - 1 = 2^a 3^b)
-  return p;
-}
-
-// The plan with an odd number of stages, for a transform that ping-pongs between the slot and the
-// spare (the first stage reads the slot and writes the spare, so the last one writes the spare
-// too): one radix-4 stage split into two radix-2 stages (the same FP64 instructions per point), or
-// two radix-2 stages merged; no stages when neither exists (N = 2 * 3^b with b odd).
-__device__ __forceinline__ RadixPlan odd_stages(RadixPlan p) {
-  if (p.stages() & 1) return p;
-  if (p.n4 > 0) return RadixPlan{p.n3, p.n4 - 1, p.n2 + 2};
-  if (p.n2 >= 2) return RadixPlan{p.n3, p.n4 + 1, p.n2 - 2};
-  return RadixPlan{0, 0, 0};
-}
-
-// Untwiddled radix-R butterfly (the first stage of an FFT).
-template <int R>
-__device__ __forceinline__ void butterfly_plain(double2* v, double2* o) {
-  if (R == 2) {
-    o[0] = cadd(v[0], v[1]);
-    o[1] = csub(v[0], v[1]);
-  } else if (R == 4) {
-    double2 a = cadd(v[0], v[2]), b = csub(v[0], v[2]);
-    double2 e = cadd(v[1], v[3]), f = csub(v[1], v[3]);
-    o[0] = cadd(a, e);
-    o[2] = csub(a, e);
-    o[1] = make_double2(b.x + f.y, b.y - f.x);  // b - i f
-    o[3] = make_double2(b.x - f.y, b.y + f.x);  // b + i f
-  } else {  // R == 3, W3 = -1/2 - i sqrt(3)/2
-    const double h = 0.86602540378443864676;
-    double2 t1 = cadd(v[1], v[2]);
-    double2 t2 = make_double2(fma(-0.5, t1.x, v[0].x), fma(-0.5, t1.y, v[0].y));
-    double2 t3 = csub(v[1], v[2]);
-    o[0] = cadd(v[0], t1);
-    o[1] = make_double2(fma(h, t3.y, t2.x), fma(-h, t3.x, t2.y));  // t2 - i h t3
-    o[2] = make_double2(fma(-h, t3.y, t2.x), fma(h, t3.x, t2.y));  // t2 + i h t3
-  }
-}
-
-// The first radix-R stage of the even DCT's FFT (Ns = 1, no twiddles) with the fold computed on
-// its way in: u_m = (x_m + x_{N-m})/2 - sin(pi m/N) (x_m - x_{N-m}) = x_{N-m} + (1/2 - sin(pi m/N))
-// (x_m - x_{N-m}), one FMA a point, of both lines of every pair, read straight from the slots (no
-// separate fold phase, one barrier fewer per transform).
-template <int R>
-__device__ __forceinline__ void fold_stage(const Ctx& c, double2* dst, const double2* tw, int N, int nall,
-                                           int npairs, int slot0, const DctScale& ds) {
-  const int c_tb = c.tb;
-  const int c_lcap = c.lcap;
-  const int c_nthreads = c.nthreads;
-  const int c_tid = c.tid;
-  const int c_fft_stride = c.fft_stride;
-  const int LR = N / R;
-  const double* cmt = reinterpret_cast<const double*>(tw + 2 * N);
-  double* const x0s = slot_ptr(c, slot0);
-  for (int idx = c_tid; idx < nall * LR; idx += c_nthreads) {
-    const int P = idx / LR, j = idx - P * LR;
-    const int sl = P / npairs, pr = P - sl * npairs;
-    const double* x = op_slot(c, x0s, slot0, sl);
-    const int t0 = 2 * pr;
-    const bool two = t0 + 1 < c_tb;
-    double2 v[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int m = j + r * LR;
-      const double cm = __ldg(cmt + m);  // 1/2 - sin(pi m / N), after the 2N twiddles
-      const double a0 = x[t0 * c_lcap + m], a1 = x[t0 * c_lcap + N - m];
-      double ua = fma(cm, a0 - a1, a1);
-      double ub = 0.0;
-      if (two) {
-        const double b0 = x[(t0 + 1) * c_lcap + m], b1 = x[(t0 + 1) * c_lcap + N - m];
-        ub = fma(cm, b0 - b1, b1);
-      }
-      if (ds.has_pre) {
-        ua = ds.scale_pre(ua, m, N);
-        ub = ds.scale_pre(ub, m, N);
-      }
-      v[r] = make_double2(ua, ub);
-    }
-    double2 o[R];
-    butterfly_plain<R>(v, o);
-#pragma unroll
-    for (int q = 0; q < R; ++q) dst[P * c_fft_stride + j * R + q] = o[q];
-  }
-}
-
+// ------------------------------------------------------------ even DCT-I
 // DCT-I for even N = n - 1, exploiting both the realness and the even symmetry
-// of the extension (half the FFT length of the paired approach):
-//   fold   u_j = (x_j + x_{N-j})/2 - sin(pi j/N) (x_j - x_{N-j}),  j = 0..N-1
-//          y_1 = (x_0 - x_N) + 2 sum_{0<j<N/2} (x_j - x_{N-j}) cos(pi j/N)
-//   FFT    Z = DFT_N(u_a + i u_b) for the two lines (a, b) of a pair
+// of the extension (half the FFT length of the paired approach), in 64-bit fixed point
+// (pgx_fixed.cuh: one scale per line):
+//   fold   u_j = (x_j + x_{N-j})/2 - sin(pi j/N) (x_j - x_{N-j}),  j = 0..N-1:
+//          u_m = x_{N-m} + p, u_{N-m} = x_m - p with p = (1/2 - sin(pi m/N)) (x_m - x_{N-m}):
+//          one product for two points
+//   FFT    Z = DFT_N(u_a + i u_b) for the two lines (a, b) of a pair; real and imaginary parts are
+//          the two lines of a buffer
 //   untangle  y_{2m} = Z_m + conj(Z_{N-m}) (real / imag part for line a / b),
 //          odd increments y_{2m+1} - y_{2m-1} = Im(Z_{N-m} - Z_m) (a), Re(Z_m - Z_{N-m}) (b)
-//   scan   y_{2m+1} = y_1 + sum of increments.
-// Every phase runs over all threads of the CTA (a barrier between phases), with the FFT's radix
-// plan (radix_plan), the fold and the per-line phases (L lanes a line) of the warp-local form.
-// tw is the table exp(-2 pi i k / (2N)): W_N^k = tw[2k], (cos, -sin)(pi j / N) = tw[j].
-// The backward pre-scale (-1)^j w_j is common to x_j and x_{N-j} (N even) and
-// applied to u_j, d_j; the forward post-scale to the outputs.
-__device__ void op_dct_even_cta(Ctx& c, const pgx_op& op, const pgx_instance& I) {
-  const int c_tb = c.tb;
-  const int c_lcap = c.lcap;
-  const int c_nthreads = c.nthreads;
-  const int c_tid = c.tid;
-  const int c_fft_stride = c.fft_stride;
-  double* const c_ybuf = c.ybuf;
-  // op.b > 1: the transforms of slots a .. a+b-1 (same length and mode) go through every
-  // phase together: one barrier per phase for all of them, b times the parallel work.
-  const int ns = nslot_of(op);
-  double* const x0s = slot_ptr(c, op.a);
-  const int n = c.slen[op.a];
-  const int N = n - 1, H = N / 2;
-  const int mode = op.k & PGX_DCT_MODE_MASK;
-  const DctScale ds = dct_scale(mode, N);
-  const double2* tw = reinterpret_cast<const double2*>(I.mat[op.mat]);
-  const int npairs = (c_tb + 1) >> 1;
-  const int nall = ns * npairs;  // line pairs of all slots; pair P = s * npairs + pr
-  int rest = 1;
-  const bool in_slot = (op.k & PGX_DCT_SLOT) != 0;
-  const RadixPlan plan = in_slot ? odd_stages(radix_plan(N, rest)) : radix_plan(N, rest);
-  if (N > c_fft_stride || rest != 1 || plan.stages() < 1 || (in_slot && (ns != 1 || (c_tb & 1)))) {
-    // no buffer or plan for this length: refuse loudly
-    for (int sl = 0; sl < ns; ++sl)
-      for (int idx = c_tid; idx < c_tb * n; idx += c_nthreads) x_nan(c, op.a + sl, idx, n);
-    return;
-  }
-  // y_1, L lanes a line, the op's lines spread over the warps (line lt = sl * tb + t); the j of a
-  // lane keep one parity (L even), so the alternating pre-scale of BWD / FWD_T is one sign per lane
-  const int nlines = ns * c_tb;
-  const LineLanes g = line_lanes(c, nlines);
-  {
-    const bool alt = mode == PGX_DCT_BWD || mode == PGX_DCT_FWD_T;
-    const double ps = ds.has_pre ? (alt ? -ds.pre(1, N) : ds.pre(1, N)) : 1.0;
-    const double p0 = ds.has_pre ? ds.pre(0, N) : 1.0;
-    for (int base = g.first; base < nlines; base += g.stride) {
-      const int lt = base + g.grp;
-      const bool valid = lt < nlines;
-      const int sl = valid ? lt / c_tb : 0, t = valid ? lt - sl * c_tb : 0;
-      const double* xl = op_slot(c, x0s, op.a, sl) + t * c_lcap;
-      double acc = 0.0;
-      if (valid)
-        for (int j = 1 + g.sub; j < H; j += g.L) acc = fma(__ldg(&tw[j].x), xl[j] - xl[N - j], acc);
-      if (alt && ((1 + g.sub) & 1)) acc = -acc;
-      for (int o = g.L >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o, g.L);
-      if (valid && g.sub == 0) c_ybuf[lt] = fma(2.0 * ps, acc, (xl[0] - xl[N]) * p0);
-    }
-  }
-  // FFT of length N over all pairs, the radix plan of the warp-local form (y_1 above and the first
-  // stage both only read the slots)
-  double2* bufs[2] = {c.f0, c.f1};
-  const int R0 = plan.at(0);
-  if (R0 == 3) fold_stage<3>(c, bufs[1], tw, N, nall, npairs, op.a, ds);
-  else if (R0 == 4) fold_stage<4>(c, bufs[1], tw, N, nall, npairs, op.a, ds);
-  else fold_stage<2>(c, bufs[1], tw, N, nall, npairs, op.a, ds);
-  int cur = 1, Ns = R0;
-  for (int s = 1; s < plan.stages(); ++s) {
-    __syncthreads();
-    stage_dispatch<false, false>(plan.at(s), c, bufs[cur], bufs[cur ^ 1], tw, N, Ns, nall, nullptr, ds, 2);
-    cur ^= 1;
-    Ns *= plan.at(s);
-  }
-  __syncthreads();
-  const double2* Z = bufs[cur];
-  // untangle: even outputs, odd increments
-  for (int idx = c_tid; idx < nall * (H + 1); idx += c_nthreads) {
-    const int P = idx / (H + 1), m = idx - P * (H + 1);
-    const int sl = P / npairs, pr = P - sl * npairs;
-    double* x = op_slot(c, x0s, op.a, sl);
-    const int t0 = 2 * pr;
-    const bool two = t0 + 1 < c_tb;
-    const double2 zm = Z[P * c_fft_stride + m];
-    const double2 zn = Z[P * c_fft_stride + (m == 0 ? 0 : N - m)];
-    double ya = zm.x + zn.x, yb = zm.y + zn.y;
-    if (ds.has_post) {
-      const double sc = ds.post(2 * m, N);
-      ya *= sc;
-      yb *= sc;
-    }
-    x[t0 * c_lcap + 2 * m] = ya;
-    if (two) x[(t0 + 1) * c_lcap + 2 * m] = yb;
-    if (m >= 1 && m < H) {
-      x[t0 * c_lcap + 2 * m + 1] = zn.y - zm.y;
-      if (two) x[(t0 + 1) * c_lcap + 2 * m + 1] = zm.x - zn.x;
-    } else if (m == 0) {
-      x[t0 * c_lcap + 1] = c_ybuf[sl * c_tb + t0];
-      if (two) x[(t0 + 1) * c_lcap + 1] = c_ybuf[sl * c_tb + t0 + 1];
-    }
-  }
-  if (in_slot) zero_tail(c, slot_ptr(c, op.a), n);  // the FFT stages wrote past the lines' ends
-  __syncthreads();
-  // odd outputs: inclusive prefix sums over k = 1, 3, ..., N-1, L lanes a line
-  {
-    const int chunk = (H + g.L - 1) / g.L;
-    const double osc = ds.has_post ? ds.post(1, N) : 1.0;  // the same for every odd k < N
-    for (int base = g.first; base < nlines; base += g.stride) {
-      const int lt = base + g.grp;
-      const bool valid = lt < nlines;
-      const int sl = valid ? lt / c_tb : 0, t = valid ? lt - sl * c_tb : 0;
-      double* xl = op_slot(c, x0s, op.a, sl) + t * c_lcap;
-      const int m0 = min(g.sub * chunk, H), m1 = min(m0 + chunk, H);
-      double run = 0.0;
-      if (valid)
-        for (int m = m0; m < m1; ++m) run += xl[2 * m + 1];
-      double incl = run;
-      for (int o = 1; o < g.L; o <<= 1) {
-        const double v = __shfl_up_sync(0xffffffffu, incl, o, g.L);
-        if (g.sub >= o) incl += v;
-      }
-      if (!valid) continue;
-      double pre = incl - run;  // exclusive prefix of this lane's chunk
-      if (ds.has_post) {
-        for (int m = m0; m < m1; ++m) {
-          pre += xl[2 * m + 1];
-          xl[2 * m + 1] = pre * osc;
-        }
-      } else {
-        for (int m = m0; m < m1; ++m) {
-          pre += xl[2 * m + 1];
-          xl[2 * m + 1] = pre;
-        }
-      }
-    }
-  }
-}
-
-// ---------------------------------------------------------- warp-local even DCT
-// The same folded half-length algorithm as op_dct_even_cta, with every phase of a line pair
-// inside one warp: warp w owns the pairs P = w, w + nw, w + 2 nw, ... of all the op's slots and
-// runs their fold, FFT stages, untangle and scan separated by __syncwarp only, so the warps of a
-// CTA (and of the other CTAs on the SM) never wait for each other inside a transform.  Per line,
-// y_1 and the odd-coefficient scan use just enough lanes to cover the warp's lines (L lanes a
-// line, log2 L shuffle steps instead of 32 lanes and 5), and the fold is one FMA per point:
-// u_m = (x_m + x_{N-m})/2 - sin(pi m/N) (x_m - x_{N-m}) = x_{N-m} + (1/2 - sin(pi m/N)) (x_m - x_{N-m}).
-
-struct WarpPairs {
-  int lane, w, nw, npw;  // lane, warp, warps of the CTA, pairs this warp owns
+//   scan   S_m, the sum of the increments up to m (integer adds, no rounding), and
+//          y_{2m+1} = S_m + y_1 with y_1 = (x_0 - x_N) - mean(S), from
+//          x_0 - x_N = (2/N) sum of the odd outputs (the transform's inverse at both ends).  Taking
+//          y_1 from the scan saves its own sum of products (one in two of the fold's), and the odd
+//          outputs keep the increments' summed errors about their mean only.
+// The twiddle table holds exp(-2 pi i k / (2N)): W_N^k = entry 2k, (cos, -sin)(pi j / N) = entry j.
+//
+// The FFT is Stockham (4, 3, 2) for any N = 2^a 3^b; the lengths that dealiased and plain grids of
+// 2^k + 1 points give, N = 2^a and 3 2^a, have builds of their own in which every length, stride and
+// division is a constant and radix 8 takes the place of a radix 4 and a radix 2 stage.  N = 3 M, M
+// a power of two, is split by the prime-factor map (n = M n1 + 3 n2, k by remainders): three
+// M-point transforms and one radix-3 pass with no twiddles between them (N = 192: 0.8 complex
+// products a point instead of 2.25).
+//
+// What bounds it: the integer multiply-adds (~5 cycles a warp each) and the instructions around them;
+// in FP64 a point took ~16 instructions of ~66 cycles.
+//
+// Two forms share the code.  Warp-local: warp w owns the pairs w, w + nw, ... of all the op's slots
+// and takes them through every phase with __syncwarp between phases.  CTA-wide: each phase's items
+// spread over all threads, block barriers between phases.
+struct FxSet {   // the pairs of the warp (warp-local) or of the CTA, and this thread's place among its threads
+  bool cta;
+  int first, step;         // items of a phase: first, first + step, ...
+  int npw, pair0, pstep;   // pair q of the set is pair0 + q * pstep
 };
-__device__ __forceinline__ WarpPairs warp_pairs(const Ctx& c, int nall) {
-  WarpPairs g;
-  g.lane = c.tid & 31;
-  g.w = c.tid >> 5;
-  g.nw = c.nthreads >> 5;
-  g.npw = g.w < nall ? (nall - g.w + g.nw - 1) / g.nw : 0;
-  return g;
+__device__ __forceinline__ void fx_sync(bool cta) {
+  if (cta) __syncthreads();
+  else __syncwarp();
 }
 
-// First stage (Ns = 1, no twiddles) with the fold on its way in, over the warp's pairs.
+// A buffer of line pairs: the real parts of pair P at p + P * pair, the imaginary parts `line` further.
+struct FxBuf {
+  int p;
+  int line, pair;
+};
+// The pairs of a multi-slot op in their slots: pair P is in slot slot0 + P / npairs (npairs < 0: one slot,
+// whose FxBuf says it all).
+struct FxSlots {
+  const Ctx* c;
+  int slot0, npairs;
+};
+__device__ __forceinline__ int64_t* fx_sm(int off) { return reinterpret_cast<int64_t*>(smem_dyn) + off; }
+__device__ __forceinline__ int64_t* fx_line(const Ctx& c, int slot, int t) {
+  return fx_sm(c.sm + (c.phys[slot] * c.tb + t) * c.lcap);
+}
+__device__ __forceinline__ int64_t* fx_pair(const FxSlots& m, const FxBuf& b, int P) {
+  if (m.npairs < 0) return fx_sm(b.p + P * b.pair);
+  int sl = 0;
+  while (P >= m.npairs) {  // a handful of slots at most
+    P -= m.npairs;
+    ++sl;
+  }
+  return fx_line(*m.c, m.slot0 + sl, 2 * P);
+}
+
+__device__ __forceinline__ fx_tw fx_table(const fx_tw* tw, int k) {
+  const int4 v = __ldg(reinterpret_cast<const int4*>(tw) + k);
+  fx_tw w;
+  w.rh = v.x; w.rl = v.y; w.ih = v.z; w.il = v.w;
+  return w;
+}
+
+// R-point DFT, no twiddles.
 template <int R>
-__device__ __forceinline__ void wfold(const Ctx& c, const WarpPairs& g, double2* dst, const double2* tw, int N,
-                                      int npairs, int slot0, const DctScale& ds) {
-  const int c_tb = c.tb;
-  const int c_lcap = c.lcap;
-  const int c_fft_stride = c.fft_stride;
-  const int B = N / R;
-  const double* cmt = reinterpret_cast<const double*>(tw + 2 * N);
-  double* const x0s = slot_ptr(c, slot0);
-  for (int it = g.lane; it < g.npw * B; it += 32) {
-    const int q = it / B, j = it - q * B;
-    const int P = g.w + q * g.nw;
-    const int sl = P / npairs, pr = P - sl * npairs;
-    const double* x = op_slot(c, x0s, slot0, sl);
-    const int t0 = 2 * pr;
-    const bool two = t0 + 1 < c_tb;
-    double2 v[R], o[R];
+__device__ __forceinline__ void fx_butterfly(const fx2* v, fx2* o) {
+  if (R == 2) {
+    o[0] = fx_add(v[0], v[1]);
+    o[1] = fx_sub(v[0], v[1]);
+  } else if (R == 3) {  // W3 = -1/2 - i sqrt(3)/2
+    const fx_w h = {929887697, -1332128537};  // sqrt(3)/2 2^62, rounded
+    const fx2 t1 = fx_add(v[1], v[2]), t3 = fx_sub(v[1], v[2]);
+    fx2 t2, ht;
+    t2.x = v[0].x - ((t1.x + 1) >> 1);
+    t2.y = v[0].y - ((t1.y + 1) >> 1);
+    ht.x = fx_mul(t3.x, h);
+    ht.y = fx_mul(t3.y, h);
+    o[0] = fx_add(v[0], t1);
+    o[1] = fx_mi(t2, ht);
+    o[2] = fx_pi(t2, ht);
+  } else if (R == 4) {
+    const fx2 a = fx_add(v[0], v[2]), b = fx_sub(v[0], v[2]);
+    const fx2 e = fx_add(v[1], v[3]), f = fx_sub(v[1], v[3]);
+    o[0] = fx_add(a, e);
+    o[2] = fx_sub(a, e);
+    o[1] = fx_mi(b, f);
+    o[3] = fx_pi(b, f);
+  } else {  // R == 8: two 4-point DFTs, of the even and the odd inputs, and W8 = (1 - i) / sqrt(2)
+    const fx_w h = {759250125, -25716447};  // sqrt(1/2) 2^62, rounded
+    fx2 e[4], f[4];
+    const fx2 ve[4] = {v[0], v[2], v[4], v[6]}, vo[4] = {v[1], v[3], v[5], v[7]};
+    fx_butterfly<4>(ve, e);
+    fx_butterfly<4>(vo, f);
+    o[0] = fx_add(e[0], f[0]);
+    o[4] = fx_sub(e[0], f[0]);
+    o[2] = fx_mi(e[2], f[2]);
+    o[6] = fx_pi(e[2], f[2]);
+    fx2 w;
+    w.x = fx_mul(f[1].x + f[1].y, h);
+    w.y = fx_mul(f[1].y - f[1].x, h);
+    o[1] = fx_add(e[1], w);
+    o[5] = fx_sub(e[1], w);
+    w.x = fx_mul(f[3].y - f[3].x, h);
+    w.y = fx_mul(f[3].x + f[3].y, h);  // W8^3 f3 = (w.x, -w.y)
+    o[3].x = e[3].x + w.x;
+    o[3].y = e[3].y - w.y;
+    o[7].x = e[3].x - w.x;
+    o[7].y = e[3].y + w.y;
+  }
+}
+
+// A line whose sum of absolute values is far above its largest one (noise, physical values) would start
+// with log2 of their ratio fewer bits than it could: the partial sums only grow to that sum stage by
+// stage.  It starts that many bits higher, and every stage shifts its results down by what is left, at
+// most its own growth.  The rounding of the first stages, which the later ones and the scan amplify,
+// then costs nothing (N = 1024, random points: 5e-14 off without it, FP64: 5e-15).  The lines of a
+// pair go down by the same bits, the larger of their two numbers: the one with fewer ends that much
+// below the scale it could have.
+constexpr int kFxGrowthN = 96;  // shorter transforms have bits to spare
+__device__ __forceinline__ int64_t fx_down(int64_t v, int sh) { return (v + ((int64_t)1 << (sh - 1))) >> sh; }
+template <int R>
+__device__ __forceinline__ void fx_shift(fx2* o, int left) {
+  if (left > 0) {
+    const int g = R > 4 ? 3 : (R > 2 ? 2 : 1);
+    const int sh = left < g ? left : g;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      const int m = j + r * B;
-      const double cm = __ldg(cmt + m);  // 1/2 - sin(pi m / N), after the 2N twiddles
-      const double a0 = x[t0 * c_lcap + m], a1 = x[t0 * c_lcap + N - m];
-      double ua = fma(cm, a0 - a1, a1);
-      double ub = 0.0;
-      if (two) {
-        const double b0 = x[(t0 + 1) * c_lcap + m], b1 = x[(t0 + 1) * c_lcap + N - m];
-        ub = fma(cm, b0 - b1, b1);
-      }
-      if (ds.has_pre) {
-        ua = ds.scale_pre(ua, m, N);
-        ub = ds.scale_pre(ub, m, N);
-      }
-      v[r] = make_double2(ua, ub);
+      o[r].x = fx_down(o[r].x, sh);
+      o[r].y = fx_down(o[r].y, sh);
     }
-    butterfly_plain<R>(v, o);
-#pragma unroll
-    for (int q2 = 0; q2 < R; ++q2) dst[P * c_fft_stride + j * R + q2] = o[q2];
   }
 }
 
-// One twiddled radix-R Stockham stage (Ns > 1) over the warp's pairs; tw holds exp(-2 pi i k / (tws L)).
-template <int R>
-__device__ __forceinline__ void wstage(const Ctx& c, const WarpPairs& g, const double2* src, double2* dst,
-                                       const double2* tw, int L, int Ns, int tws) {
-  const int c_fft_stride = c.fft_stride;
-  const int B = L / R;
-  const int step = tws * (L / (Ns * R));
-  for (int it = g.lane; it < g.npw * B; it += 32) {
-    const int q = it / B, j = it - q * B;
-    const int P = g.w + q * g.nw;
-    const int k = j % Ns;
-    const double2* s = src + P * c_fft_stride;
-    double2 v[R], o[R];
+// The scales of an op's lines, two int32 a pair from double `scales` of the shared memory: kx, and in the
+// top byte the bits the line starts above the scale of its sum.
+__device__ __forceinline__ int32_t* fx_scales(int scales) { return reinterpret_cast<int32_t*>(smem_dyn + scales); }
+__device__ __forceinline__ int fx_bits_of(int scales, int P) {
+  return max(fx_scales(scales)[2 * P] >> 24, fx_scales(scales)[2 * P + 1] >> 24);
+}
+// The scale of a line's results (word w) in a pair that went down by `down` bits.
+__device__ __forceinline__ int fx_kx_out(int32_t w, int down) { return (w & 0xffffff) + down - (w >> 24); }
+
+// One radix-R Stockham stage of any length (FIRST: Ns = 1, no twiddles); grown: bits shifted before.
+template <int R, bool FIRST>
+__device__ __forceinline__ void fx_stage(const FxSlots& m, const FxSet& g, const FxBuf& src, const FxBuf& dst,
+                                         const fx_tw* tw, int scales, int N, int Ns, int grown) {
+  const int B = N / R;
+  const FastDiv fb(B), fn(FIRST ? 1 : Ns);
+  const int step = FIRST ? 0 : 2 * fn.div(B);
+  const int total = g.npw * B;
+  for (int it = g.first; it < total; it += g.step) {
+    const int q = fb.div(it), j = it - q * B;
+    const int P = g.pair0 + q * g.pstep;
+    const int k = FIRST ? 0 : j - fn.div(j) * Ns;
+    const int64_t* s = FIRST ? fx_pair(m, src, P) : fx_sm(src.p + P * src.pair);
+    fx2 v[R], o[R];
 #pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = s[j + r * B];
-    if (R == 2) {
-      const double2 w1 = __ldg(tw + k * step);
-      o[0] = cmadd(v[0], w1, v[1]);
-      o[1] = ctwice_minus(v[0], o[0]);
-    } else if (R == 4) {
-      const double2 w1 = __ldg(tw + k * step), w2 = __ldg(tw + 2 * k * step);
-      const double2 a = cmadd(v[0], w2, v[2]), b = ctwice_minus(v[0], a);
-      const double2 cc = cmadd(v[1], w2, v[3]), d = ctwice_minus(v[1], cc);
-      o[0] = cmadd(a, w1, cc);
-      o[2] = ctwice_minus(a, o[0]);
-      o[1] = cmadd(b, make_double2(w1.y, -w1.x), d);
-      o[3] = ctwice_minus(b, o[1]);
+    for (int r = 0; r < R; ++r) {
+      v[r].x = s[j + r * B];
+      v[r].y = s[src.line + j + r * B];
+    }
+    if (!FIRST) {
+#pragma unroll
+      for (int r = 1; r < R; ++r) v[r] = fx_cmul(v[r], fx_table(tw, r * k * step));
+    }
+    fx_butterfly<R>(v, o);
+    if (N >= kFxGrowthN) fx_shift<R>(o, fx_bits_of(scales, P) - grown);
+    int64_t* t = fx_sm(dst.p + P * dst.pair) + (j - k) * R + k;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      t[r * Ns] = o[r].x;
+      t[dst.line + r * Ns] = o[r].y;
+    }
+  }
+}
+
+// The same with every length a constant: PL planes (the prime-factor columns) of M points, stage of
+// radix R at stride Ns.
+template <int R, int M, int Ns, int PL, int GROWN>
+__device__ __forceinline__ void fx_stage_n(const FxSlots& m, const FxSet& g, const FxBuf& src, const FxBuf& dst,
+                                           const fx_tw* tw, int scales) {
+  constexpr int N = M * PL, B = M / R;
+  const int total = g.npw * (PL * B);
+  for (int it = g.first; it < total; it += g.step) {
+    const int q = it / (PL * B), rem = it - q * (PL * B);
+    const int pl = PL > 1 ? rem / B : 0, j = rem - pl * B;
+    const int P = g.pair0 + q * g.pstep;
+    const int k = j & (Ns - 1);
+    const int64_t* s = (Ns == 1 && PL == 1 ? fx_pair(m, src, P) : fx_sm(src.p + P * src.pair)) + pl * M + j;
+    fx2 v[R], o[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      v[r].x = s[r * B];
+      v[r].y = s[src.line + r * B];
+    }
+    if (Ns > 1) {
+#pragma unroll
+      for (int r = 1; r < R; ++r) v[r] = fx_cmul(v[r], fx_table(tw, r * k * (2 * N / (Ns * R))));
+    }
+    fx_butterfly<R>(v, o);
+    if (N >= kFxGrowthN) fx_shift<R>(o, fx_bits_of(scales, P) - GROWN);
+    int64_t* t = fx_sm(dst.p + P * dst.pair) + pl * M + (j - k) * R + k;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      t[r * Ns] = o[r].x;
+      t[dst.line + r * Ns] = o[r].y;
+    }
+  }
+}
+
+// First pass of N = 3 M: 3-point DFTs over n1 of the points (M n1 + 3 n2) mod N, results to plane k1.
+template <int M>
+__device__ __forceinline__ void fx_stage_3(const FxSlots& m, const FxSet& g, const FxBuf& src, const FxBuf& dst,
+                                           int scales) {
+  constexpr int N = 3 * M;
+  const int total = g.npw * M;
+  for (int it = g.first; it < total; it += g.step) {
+    const int q = it / M, n2 = it - q * M;
+    const int P = g.pair0 + q * g.pstep;
+    const int64_t* s = fx_pair(m, src, P);
+    const int i0 = 3 * n2, i1 = i0 + M < N ? i0 + M : i0 + M - N, i2 = i1 + M < N ? i1 + M : i1 + M - N;
+    fx2 v[3], o[3];
+    v[0].x = s[i0];
+    v[0].y = s[src.line + i0];
+    v[1].x = s[i1];
+    v[1].y = s[src.line + i1];
+    v[2].x = s[i2];
+    v[2].y = s[src.line + i2];
+    fx_butterfly<3>(v, o);
+    if (N >= kFxGrowthN) fx_shift<3>(o, fx_bits_of(scales, P));
+    int64_t* t = fx_sm(dst.p + P * dst.pair) + n2;
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      t[r * M] = o[r].x;
+      t[dst.line + r * M] = o[r].y;
+    }
+  }
+}
+
+__host__ __device__ constexpr int fx_log2(int m) { return m > 1 ? 1 + fx_log2(m / 2) : 0; }
+// The M-point stages of a plan, ping-pong: src -> dst, then dst -> other, other -> dst, ...; returns the
+// offset of the buffer that holds the result.
+template <int M, int PL, int Ns, int GROWN>
+__device__ __forceinline__ int fx_stages(const FxSlots& m, const FxSet& g, const FxBuf& src, const FxBuf& dst,
+                                         const FxBuf& other, const fx_tw* tw, int scales) {
+  if constexpr (Ns == M) {
+    return src.p;
+  } else {
+    // fours until what is left is a power of eight: the rounding of a stage grows with the stages after
+    // it, and the lines are at their final scale by the last ones
+    constexpr int R = fx_log2(M / Ns) % 3 == 0 ? 8 : 4;
+    fx_stage_n<R, M, Ns, PL, GROWN>(m, g, src, dst, tw, scales);
+    fx_sync(g.cta);
+    return fx_stages<M, PL, Ns * R, GROWN + (R == 8 ? 3 : 2)>(m, g, dst, other, dst, tw, scales);
+  }
+}
+template <int N>
+__device__ __forceinline__ int fx_fft_n(const FxSlots& m, const FxSet& g, const FxBuf& src, const FxBuf& b0,
+                                        const FxBuf& b1, const fx_tw* tw, int scales) {
+  if constexpr (N % 3 == 0) {
+    fx_stage_3<N / 3>(m, g, src, b1, scales);
+    fx_sync(g.cta);
+    return fx_stages<N / 3, 3, 1, 2>(m, g, b1, b0, b1, tw, scales);
+  } else {
+    return fx_stages<N, 1, 1, 0>(m, g, src, b1, b0, tw, scales);
+  }
+}
+
+// Radix plan of any other length: every factor 3 first, then 4s, then one 2.
+__device__ __forceinline__ int fx_fft_any(const FxSlots& m, const FxSet& g, FxBuf src, FxBuf b0, FxBuf b1,
+                                          const fx_tw* tw, int scales, int N) {
+  int rest = N, Ns = 1, grown = 0;
+  FxBuf dst = b1;
+  while (rest > 1) {
+    const int R = rest % 3 == 0 ? 3 : ((rest & 3) == 0 ? 4 : 2);
+    if (Ns == 1) {
+      if (R == 3) fx_stage<3, true>(m, g, src, dst, tw, scales, N, 1, 0);
+      else if (R == 4) fx_stage<4, true>(m, g, src, dst, tw, scales, N, 1, 0);
+      else fx_stage<2, true>(m, g, src, dst, tw, scales, N, 1, 0);
     } else {
-      if (k != 0) {
-        v[1] = cmul(v[1], __ldg(tw + k * step));
-        v[2] = cmul(v[2], __ldg(tw + 2 * k * step));
-      }
-      butterfly_plain<3>(v, o);
+      if (R == 3) fx_stage<3, false>(m, g, src, dst, tw, scales, N, Ns, grown);
+      else if (R == 4) fx_stage<4, false>(m, g, src, dst, tw, scales, N, Ns, grown);
+      else fx_stage<2, false>(m, g, src, dst, tw, scales, N, Ns, grown);
     }
-    double2* d = dst + P * c_fft_stride + (j - k) * R + k;
-#pragma unroll
-    for (int q2 = 0; q2 < R; ++q2) d[q2 * Ns] = o[q2];
+    fx_sync(g.cta);
+    grown += R > 2 ? 2 : 1;
+    Ns *= R;
+    rest /= R;
+    src = dst;
+    dst = dst.p == b1.p ? b0 : b1;
   }
+  return src.p;
 }
 
-__device__ void op_dct_even(Ctx& c, const pgx_op& op, const pgx_instance& I) {
-  const int c_tb = c.tb;
-  const int c_lcap = c.lcap;
-  const int c_nthreads = c.nthreads;
-  const int c_tid = c.tid;
-  const int c_fft_stride = c.fft_stride;
-  double* const c_ybuf = c.ybuf;
+// Sum of absolute values of a line (n points), this lane's share, in FP32 over the high words (the low
+// ones add less than 2^-20 of it): the double's exponent field moves into the float's, `shift` further
+// down, clamped at zero and near the top.
+__device__ __forceinline__ uint32_t fx_hi(const int64_t* x, int j) {
+  return (uint32_t)((uint64_t)x[j] >> 32) & 0x7fffffffu;
+}
+__device__ __forceinline__ float fx_abs_part(uint32_t hi, int shift) {
+  return __int_as_float(__viaddmin_s32_relu((int)hi, -shift, 254 << 20) << 3);
+}
+struct FxScale {
+  int kx;    // FX_KX0 + q with the line's sum of absolute values below 2^q; FX_BAD, FX_ZERO
+  int bits;  // q less the exponent of a power of two above every value, at least 0
+};
+// Scale of a line shared by a group of L lanes.  Sums outside [2^-60, 2^100] are taken again relative
+// to the largest exponent.
+// ends2: with the end points counted twice (the modes that halve every other point run on doubled ends
+// and half the scale).
+__device__ __forceinline__ FxScale fx_line_scale(const int64_t* x, int n, const LineLanes& g, bool ends2,
+                                                 bool valid, bool growth) {
+  float f = 0.0f;
+  uint32_t hm = 0;
+  int r = 0;
+  if (valid) {
+    for (int j = g.sub; j < n; j += g.L) {
+      const uint32_t h = fx_hi(x, j);
+      f += fx_abs_part(h, 896 << 20);
+      if (growth) hm = max(hm, h);
+    }
+    if (ends2 && g.sub < 2) f += fx_abs_part(fx_hi(x, g.sub ? n - 1 : 0), 896 << 20);
+  }
+  for (int o = g.L >> 1; o > 0; o >>= 1) {
+    f += __shfl_xor_sync(FULLMASK, f, o, g.L);
+    if (growth) hm = max(hm, __shfl_xor_sync(FULLMASK, hm, o, g.L));
+  }
+  FxScale sc;
+  if (__any_sync(FULLMASK, valid && !(f >= 0x1p-60f && f <= 0x1p100f))) {
+    hm = 0;
+    uint32_t any = 0;
+    if (valid)
+      for (int j = g.sub; j < n; j += g.L) {
+        hm = max(hm, fx_hi(x, j));
+        any |= fx_hi(x, j) | (uint32_t)x[j];
+      }
+    for (int o = g.L >> 1; o > 0; o >>= 1) {
+      hm = max(hm, __shfl_xor_sync(FULLMASK, hm, o, g.L));
+      any |= __shfl_xor_sync(FULLMASK, any, o, g.L);
+    }
+    const int e = max((int)(hm >> 20), 1);
+    f = 0.0f;
+    if (valid) {
+      for (int j = g.sub; j < n; j += g.L) f += fx_abs_part(fx_hi(x, j), (e - 127) << 20);
+      if (ends2 && g.sub < 2) f += fx_abs_part(fx_hi(x, g.sub ? n - 1 : 0), (e - 127) << 20);
+    }
+    for (int o = g.L >> 1; o > 0; o >>= 1) f += __shfl_xor_sync(FULLMASK, f, o, g.L);
+    r = e - 1023;
+    if (hm >= 0x7ff00000u || any == 0) {
+      sc.kx = any ? FX_BAD : FX_ZERO;
+      sc.bits = 0;
+      return sc;
+    }
+  }
+  const int q = fx_exponent(f, r);
+  sc.kx = max(FX_KX0 + q, (int)FX_KX_MIN);
+  // the largest value is below 2^(e - 1022) for its exponent field e (doubled ends: twice that)
+  sc.bits = growth ? max(q + 1022 - max((int)(hm >> 20), 1) - (ends2 ? 1 : 0), 0) : 0;
+  return sc;
+}
+
+// The diagonal scalings of a mode around the raw transform (see DctScale), as the integer form needs
+// them: input signs (-1)^j, doubled ends (with half the scale), output times 1/N, halved ends, signs.
+struct FxMode {
+  bool alt_in, ends_in, inv_out, alt_out;
+};
+__device__ __forceinline__ FxMode fx_mode(int mode) {
+  FxMode m;
+  m.alt_in = mode == PGX_DCT_BWD || mode == PGX_DCT_FWD_T;
+  m.ends_in = mode == PGX_DCT_BWD || mode == PGX_DCT_BWD_T;
+  m.inv_out = mode == PGX_DCT_FWD || mode == PGX_DCT_FWD_T;  // ends half as much; FWD_T: (1/2N) in times 1 or 2 out
+  m.alt_out = mode == PGX_DCT_FWD || mode == PGX_DCT_BWD_T;
+  return m;
+}
+// Output y of a line of scale kx, times 2^p, as the bits of a double: the lines are read and written as
+// 64-bit integers throughout
+__device__ __forceinline__ int64_t fx_out(int64_t y, int kx, int p, bool mul, fx_w inv) {
+  if (mul) y = fx_mul(y, inv);
+  const int64_t r = (int64_t)fx_bits(fx_to_double(y, p + kx));
+  // the special scales plus the pair's bits stay above FX_BAD; a NaN line, then a line of zeros
+  return kx >= FX_BAD ? (kx >= FX_ZERO ? 0 : 0x7ff8000000000000LL) : r;
+}
+
+// Line ll of the set's lines: slot offset sl and line t of the tile; false past the end.
+__device__ __forceinline__ bool fx_line_of(const FxSet& g, int ll, int lines, int tb, int npairs, int& sl, int& t) {
+  sl = t = 0;
+  if (ll >= lines) return false;
+  if (g.cta) {
+    sl = 0;
+    t = ll;
+    while (t >= tb) {
+      t -= tb;
+      ++sl;
+    }
+    return true;
+  }
+  int pr = g.pair0 + (ll >> 1) * g.pstep;  // warp-local: line (ll & 1) of the warp's pair ll / 2
+  while (pr >= npairs) {
+    pr -= npairs;
+    ++sl;
+  }
+  t = 2 * pr + (ll & 1);
+  if (t < tb) return true;
+  t = 0;
+  return false;
+}
+
+__device__ __forceinline__ void op_dct_even(Ctx& c, const pgx_op& op, const double* table) {
+  // op.b > 1: the transforms of slots a .. a+b-1 (same length and mode) go through every
+  // phase together: one barrier per phase for all of them, b times the parallel work.
+  const int tb = c.tb, lcap = c.lcap, slot0 = op.a;
   const int ns = nslot_of(op);
-  double* const x0s = slot_ptr(c, op.a);
-  const int n = c.slen[op.a];
-  const int N = n - 1, H = N / 2;
-  const int mode = op.k & PGX_DCT_MODE_MASK;
-  const DctScale ds = dct_scale(mode, N);
-  const double2* tw = reinterpret_cast<const double2*>(I.mat[op.mat]);
-  const int npairs = (c_tb + 1) >> 1;
+  const int npairs = (tb + 1) >> 1;
   const int nall = ns * npairs;  // line pairs of all slots; pair P = s * npairs + pr
-  int rest = 1;
+  const int n = c.slen[slot0];
+  const int N = n - 1, H = N / 2;
+  const FxMode md = fx_mode(op.k & PGX_DCT_MODE_MASK);
   const bool in_slot = (op.k & PGX_DCT_SLOT) != 0;
-  const RadixPlan plan = radix_plan(N, rest);
-  if (N > c_fft_stride || rest != 1 || plan.stages() < 1 ||
-      (in_slot && (ns != 1 || (c_tb & 1) || odd_stages(plan).stages() < 1))) {
+  const bool odd_tile = (tb & 1) != 0;
+  // N = 2^a 3^b; in the slot (the contract of PGX_DCT_SLOT) not 2 3^b with odd b
+  int rest = N >> (__ffs(N) - 1), b3 = 0;
+  while (rest % 3 == 0) {
+    rest /= 3;
+    ++b3;
+  }
+  if (N > c.fft_stride || rest != 1 || (in_slot && (ns != 1 || odd_tile || ((N & 3) == 2 && (b3 & 1))))) {
     // no buffer or plan for this length: refuse loudly
     for (int sl = 0; sl < ns; ++sl)
-      for (int idx = c_tid; idx < c_tb * n; idx += c_nthreads) x_nan(c, op.a + sl, idx, n);
+      for (int idx = c.tid; idx < tb * n; idx += c.nthreads) x_nan(c, slot0 + sl, idx, n);
     return;
   }
-  const WarpPairs g = warp_pairs(c, nall);
-  if (g.npw == 0) return;
-  // A radix-4 stage and two radix-2 stages issue the same FP64 instructions per point, but the
-  // warp's butterfly count per stage (npw N / R) leaves different numbers of lanes idle in its last
-  // iteration: take radix 2 where that needs fewer FP64 warp instructions (6 per radix-2 butterfly
-  // and level, 24 per radix-4 butterfly and two levels).
-  RadixPlan wplan = 6 * ((g.npw * N + 63) >> 6) < 12 * ((g.npw * N + 127) >> 7) ? radix_plan(N, rest, true) : plan;
-  if (in_slot) wplan = odd_stages(wplan);  // the last stage writes the spare, not the slot
-  const int nl = 2 * g.npw;  // lines of the warp's pairs (the last one of an odd tile may not exist)
-  const int L = lanes_per_line(nl), per = 32 / L, grp = g.lane / L, sub = g.lane & (L - 1);
+  // a tile with fewer line pairs per slot than warps (single instances, short passes) would leave warps
+  // idle in the warp-local form (per slot, so a multi-slot op and its one-op-per-slot split agree)
+  FxSet g;
+  LineLanes ln;
+  const int lane = c.tid & 31, w = c.tid >> 5, nw = c.nthreads >> 5;
+  int lines;
+  g.cta = (op.k & PGX_DCT_CTA) || npairs < nw;
+  if (g.cta) {
+    g.first = c.tid;
+    g.step = c.nthreads;
+    g.npw = nall;
+    g.pair0 = 0;
+    g.pstep = 1;
+    lines = ns * tb;
+    ln = line_lanes(c, lines);
+  } else {
+    g.first = lane;
+    g.step = 32;
+    g.npw = w < nall ? (nall - w + nw - 1) / nw : 0;
+    g.pair0 = w;
+    g.pstep = nw;
+    lines = 2 * g.npw;
+    ln.L = lanes_per_line(max(lines, 1));
+    ln.per = 32 / ln.L;
+    ln.grp = lane / ln.L;
+    ln.sub = lane & (ln.L - 1);
+    ln.first = 0;
+    ln.stride = ln.per;
+  }
+  // the table: 2N complex doubles, N doubles, then 2N fixed-point entries and the one of 1/N
+  const fx_tw* tw = reinterpret_cast<const fx_tw*>(table + 5 * N);
+  // f0, f1: separate buffers, or the slot and the spare (lines of fft_stride = lcap points)
+  const int scales = c.ybuf, line = c.fft_stride;
+  const FxBuf b0 = {c.f0, line, 2 * line}, b1 = {c.f1, line, 2 * line};
+  int32_t* const kxs = fx_scales(scales);  // line t of slot offset sl: 2 (sl * npairs) + t
 
-  // y_1, L lanes a line: the j of a lane keep one parity (L even), so the alternating pre-scale
-  // of BWD / FWD_T is one sign per lane
-  {
-    const bool alt = mode == PGX_DCT_BWD || mode == PGX_DCT_FWD_T;
-    const double ps = ds.has_pre ? (alt ? -ds.pre(1, N) : ds.pre(1, N)) : 1.0;
-    const double p0 = ds.has_pre ? ds.pre(0, N) : 1.0;
-    for (int base = 0; base < nl; base += per) {
-      const int ll = base + grp, q = ll >> 1;
-      const int P = g.w + q * g.nw;
-      const int sl = P / npairs, t = 2 * (P - sl * npairs) + (ll & 1);
-      const bool valid = ll < nl && t < c_tb;
-      double acc = 0.0;
-      const double* xl = op_slot(c, x0s, op.a, valid ? sl : 0) + (valid ? t : 0) * c_lcap;
-      if (valid)
-        for (int j = 1 + sub; j < H; j += L) acc = fma(__ldg(&tw[j].x), xl[j] - xl[N - j], acc);
-      if (alt && ((1 + sub) & 1)) acc = -acc;
-      for (int o = L >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o, L);
-      if (valid && sub == 0) c_ybuf[sl * c_tb + t] = fma(2.0 * ps, acc, (xl[0] - xl[N]) * p0);
+  const bool growth = N >= kFxGrowthN;
+  if (growth) {  // the lines of a pair depend on each other's bits: all scales first
+    for (int base = ln.first; base < lines; base += ln.stride) {
+      int sl, t;
+      const bool valid = fx_line_of(g, base + ln.grp, lines, tb, npairs, sl, t);
+      const FxScale k = fx_line_scale(fx_line(c, slot0 + sl, t), n, ln, md.ends_in, valid, true);
+      // two bits stay: a pair then starts below 2^58, the sums of four that a radix-8 stage multiplies
+      // stay below 2^60.5 and its results, before their shift, below 2^61
+      const int word = k.kx | ((k.kx > 64 ? max(k.bits - 2, 0) : 0) << 24);
+      if (valid && ln.sub == 0) {
+        kxs[2 * sl * npairs + t] = word;
+        if (odd_tile && t == tb - 1) kxs[2 * sl * npairs + t + 1] = word;  // the missing line
+      }
     }
+    fx_sync(g.cta);
   }
-  // FFT of length N over the warp's pairs, ping-pong between the two buffers
-  double2* bufs[2] = {c.f0, c.f1};
-  const int R0 = wplan.at(0);
-  if (R0 == 3) wfold<3>(c, g, bufs[1], tw, N, npairs, op.a, ds);
-  else if (R0 == 4) wfold<4>(c, g, bufs[1], tw, N, npairs, op.a, ds);
-  else wfold<2>(c, g, bufs[1], tw, N, npairs, op.a, ds);
-  int cur = 1, Ns = R0;
-  for (int s = 1; s < wplan.stages(); ++s) {
+  // scale and fold, L lanes a line: lines in place in their slots (a tile of an odd number of
+  // lines has no room there for its last pair: into f0, the missing line zero).  x_0 - x_N waits in
+  // the line's point N, which the FFT does not use.
+  for (int base = ln.first; base < lines; base += ln.stride) {
+    int sl, t;
+    const bool valid = fx_line_of(g, base + ln.grp, lines, tb, npairs, sl, t);
+    int64_t* x = fx_line(c, slot0 + sl, t);
+    const int P = sl * npairs + (t >> 1);
+    int kx, bits = 0, down = 0;
+    if (growth) {
+      kx = kxs[2 * P + (t & 1)] & 0xffffff;
+      bits = kxs[2 * P + (t & 1)] >> 24;
+      down = fx_bits_of(scales, P);
+    } else {
+      kx = fx_line_scale(x, n, ln, md.ends_in, valid, false).kx;
+      if (valid && ln.sub == 0) kxs[2 * P + (t & 1)] = kx;
+    }
     __syncwarp();
-    const int R = wplan.at(s);
-    if (R == 4) wstage<4>(c, g, bufs[cur], bufs[cur ^ 1], tw, N, Ns, 2);
-    else if (R == 2) wstage<2>(c, g, bufs[cur], bufs[cur ^ 1], tw, N, Ns, 2);
-    else wstage<3>(c, g, bufs[cur], bufs[cur ^ 1], tw, N, Ns, 2);
-    cur ^= 1;
-    Ns *= R;
-  }
-  __syncwarp();
-  const double2* Z = bufs[cur];
-  // untangle: even outputs, odd increments (y_1 from the y_1 phase)
-  for (int it = g.lane; it < g.npw * (H + 1); it += 32) {
-    const int q = it / (H + 1), m = it - q * (H + 1);
-    const int P = g.w + q * g.nw;
-    const int sl = P / npairs, pr = P - sl * npairs;
-    double* x = op_slot(c, x0s, op.a, sl);
-    const int t0 = 2 * pr;
-    const bool two = t0 + 1 < c_tb;
-    const double2 zm = Z[P * c_fft_stride + m];
-    const double2 zn = Z[P * c_fft_stride + (m == 0 ? 0 : N - m)];
-    double ya = zm.x + zn.x, yb = zm.y + zn.y;
-    if (ds.has_post) {
-      const double sc = ds.post(2 * m, N);
-      ya *= sc;
-      yb *= sc;
-    }
-    x[t0 * c_lcap + 2 * m] = ya;
-    if (two) x[(t0 + 1) * c_lcap + 2 * m] = yb;
-    if (m >= 1 && m < H) {
-      x[t0 * c_lcap + 2 * m + 1] = zn.y - zm.y;
-      if (two) x[(t0 + 1) * c_lcap + 2 * m + 1] = zm.x - zn.x;
-    } else if (m == 0) {
-      x[t0 * c_lcap + 1] = c_ybuf[sl * c_tb + t0];
-      if (two) x[(t0 + 1) * c_lcap + 1] = c_ybuf[sl * c_tb + t0 + 1];
+    if (!valid) continue;
+    int64_t* u = odd_tile ? fx_sm(b0.p + P * b0.pair + (t & 1) * line) : x;
+    const bool fill = odd_tile && t == tb - 1;  // the last pair's missing line
+    // a line with a NaN or an infinity, or without any number: every point zero until the end
+    const int kc = kx >= FX_BAD ? FX_KX0 + 4096 : kx - bits;
+    for (int m = ln.sub; m <= H; m += ln.L) {
+      const int neg = md.alt_in && (m & 1), dbl = md.ends_in && m == 0;
+      const int64_t a = fx_from_double(fx_double((uint64_t)x[m]), kc, neg, dbl);
+      const int64_t b = fx_from_double(fx_double((uint64_t)x[N - m]), kc, neg, dbl);
+      const fx_tw e = fx_table(tw, m);
+      const int64_t df = a - b;
+      const int64_t p = fx_mul(df, fx_w{e.ih + (1 << 29), e.il});  // 1/2 - sin(pi m / N)
+      u[m] = b + p;
+      if (fill) u[line + m] = 0;
+      if (m > 0) {
+        u[N - m] = a - p;
+        if (fill) u[line + N - m] = 0;
+      } else {  // point N is no input of the FFT
+        x[N] = down ? fx_down(df, down) : df;
+      }
     }
   }
-  if (in_slot) {  // the FFT stages wrote past the ends of the warp's lines: zero [n, lcap) again
-    const int w = c_lcap - n;
-    double* x = slot_ptr(c, op.a);
-    for (int it = g.lane; it < g.npw * 2 * w; it += 32) {
-      const int q = it / (2 * w), r = it - q * 2 * w;
-      const int t = 2 * (g.w + q * g.nw) + (r >= w ? 1 : 0);  // one slot: pair P = line pair P
-      x[t * c_lcap + n + (r >= w ? r - w : r)] = 0.0;
-    }
+  fx_sync(g.cta);
+  // FFT of length N over the pairs
+  const FxSlots ms = {&c, slot0, ns == 1 || odd_tile ? -1 : npairs};
+  const FxBuf src = odd_tile ? b0 : FxBuf{c.sm + c.phys[slot0] * tb * lcap, lcap, 2 * lcap};
+  int zp;
+  switch (N) {
+    case 16: zp = fx_fft_n<16>(ms, g, src, b0, b1, tw, scales); break;
+    case 24: zp = fx_fft_n<24>(ms, g, src, b0, b1, tw, scales); break;
+    case 32: zp = fx_fft_n<32>(ms, g, src, b0, b1, tw, scales); break;
+    case 48: zp = fx_fft_n<48>(ms, g, src, b0, b1, tw, scales); break;
+    case 64: zp = fx_fft_n<64>(ms, g, src, b0, b1, tw, scales); break;
+    case 96: zp = fx_fft_n<96>(ms, g, src, b0, b1, tw, scales); break;
+    case 128: zp = fx_fft_n<128>(ms, g, src, b0, b1, tw, scales); break;
+    case 192: zp = fx_fft_n<192>(ms, g, src, b0, b1, tw, scales); break;
+    case 256: zp = fx_fft_n<256>(ms, g, src, b0, b1, tw, scales); break;
+    case 384: zp = fx_fft_n<384>(ms, g, src, b0, b1, tw, scales); break;
+    case 512: zp = fx_fft_n<512>(ms, g, src, b0, b1, tw, scales); break;
+    case 768: zp = fx_fft_n<768>(ms, g, src, b0, b1, tw, scales); break;
+    case 1024: zp = fx_fft_n<1024>(ms, g, src, b0, b1, tw, scales); break;
+    default: zp = fx_fft_any(ms, g, src, b0, b1, tw, scales, N); break;
   }
-  __syncwarp();
-  // odd outputs: inclusive prefix sums over k = 1, 3, ..., N-1, L lanes a line
+  // the planes of the prime-factor builds: k is in plane k mod 3 of M = N / 3 points, place k mod M
+  const int M = b3 == 1 && (N & 7) == 0 && N <= 768 ? N / 3 : 0;
+  const fx_tw ie = fx_table(tw, 2 * N);
+  const fx_w inv = {ie.rh, ie.rl};
+  const bool mul = md.inv_out && (inv.l != 0 || inv.h != (1 << 30));  // N not a power of two
+  const int p0 = (md.ends_in ? -1 : 0) - (md.inv_out ? ie.ih : 0) - FX_P0;
+  // a result in the slot itself (an even number of stages there): the outputs go to the spare, which
+  // becomes the slot
+  const bool swap = in_slot && zp == b0.p;
+  // untangle: even outputs, odd increments (integers until the scan)
   {
-    const int chunk = (H + L - 1) / L;
-    const double osc = ds.has_post ? ds.post(1, N) : 1.0;  // the same for every odd k < N
-    for (int base = 0; base < nl; base += per) {
-      const int ll = base + grp, q = ll >> 1;
-      const int P = g.w + q * g.nw;
-      const int sl = P / npairs, t = 2 * (P - sl * npairs) + (ll & 1);
-      const bool valid = ll < nl && t < c_tb;
-      double* xl = op_slot(c, x0s, op.a, valid ? sl : 0) + (valid ? t : 0) * c_lcap;
-      const int m0 = min(sub * chunk, H), m1 = min(m0 + chunk, H);
-      double run = 0.0;
-      if (valid)
-        for (int m = m0; m < m1; ++m) run += xl[2 * m + 1];
-      double incl = run;
-      for (int o = 1; o < L; o <<= 1) {
-        const double v = __shfl_up_sync(0xffffffffu, incl, o, L);
-        if (sub >= o) incl += v;
+    const FastDiv fh(H + 1);
+    const int total = g.npw * (H + 1);
+    for (int it = g.first; it < total; it += g.step) {
+      const int q = fh.div(it), m = it - q * (H + 1);
+      const int P = g.pair0 + q * g.pstep;
+      int sl = 0, pr = P;
+      while (pr >= npairs) {
+        pr -= npairs;
+        ++sl;
       }
-      if (!valid) continue;
-      double pre = incl - run;  // exclusive prefix of this lane's chunk
-      if (ds.has_post) {
-        for (int m = m0; m < m1; ++m) {
-          pre += xl[2 * m + 1];
-          xl[2 * m + 1] = pre * osc;
-        }
-      } else {
-        for (int m = m0; m < m1; ++m) {
-          pre += xl[2 * m + 1];
-          xl[2 * m + 1] = pre;
-        }
+      const int64_t* z = fx_sm(zp + P * b0.pair);
+      int64_t* x = fx_line(c, slot0 + sl, 2 * pr);
+      int64_t* y = swap ? fx_sm(b1.p + 2 * pr * lcap) : x;
+      const bool two = 2 * pr + 1 < tb;
+      int im = m, in = m == 0 ? 0 : N - m;
+      if (M) {
+        const int r3 = m % 3;
+        im = r3 * M + (m & (M - 1));
+        in = (r3 == 0 ? 0 : (3 - r3) * M) + ((0 - m) & (M - 1));
       }
+      const int64_t zmx = z[im], zmy = z[line + im], znx = z[in], zny = z[line + in];
+      const int pe = p0 - (md.inv_out && (m == 0 || m == H) ? 1 : 0);
+      const int down = growth ? fx_bits_of(scales, P) : 0;
+      const int ka = fx_kx_out(kxs[2 * P], down), kb = fx_kx_out(kxs[2 * P + 1], down);
+      if (m == H) {  // x_0 - x_N, which waited in point N
+        y[1] = x[N];
+        if (two) y[lcap + 1] = x[lcap + N];
+      } else if (m > 0) {
+        y[2 * m + 1] = zny - zmy;
+        if (two) y[lcap + 2 * m + 1] = zmx - znx;
+      }
+      y[2 * m] = fx_out(zmx + znx, ka, pe, mul, inv);
+      if (two) y[lcap + 2 * m] = fx_out(zmy + zny, kb, pe, mul, inv);
+    }
+  }
+  if (swap) {
+    swap_spare(c, slot0);
+    zero_tail(c, slot_ptr(c, slot0), n);
+  }
+  fx_sync(g.cta);
+  // odd outputs, L lanes a line: S_m and its sum over the line, exactly, in two 64-bit halves
+  const int chunk = (H + ln.L - 1) / ln.L;
+  for (int base = ln.first; base < lines; base += ln.stride) {
+    int sl, t;
+    const bool valid = fx_line_of(g, base + ln.grp, lines, tb, npairs, sl, t);
+    int64_t* x = fx_line(c, slot0 + sl, t);
+    const int m0 = min(ln.sub * chunk, H), m1 = valid ? min(m0 + chunk, H) : m0;
+    int64_t run = 0, hi = 0, lo = 0;
+    for (int m = m0; m < m1; ++m) {
+      if (m > 0) run += x[2 * m + 1];
+      hi += run >> 32;
+      lo += (int64_t)(uint32_t)run;
+    }
+    int64_t incl = run;
+    for (int o = 1; o < ln.L; o <<= 1) {
+      const int64_t v = __shfl_up_sync(FULLMASK, incl, o, ln.L);
+      if (ln.sub >= o) incl += v;
+    }
+    int64_t pre = incl - run;  // sum of the increments before this lane's
+    hi += (pre >> 32) * (m1 - m0);
+    lo += (int64_t)(uint32_t)pre * (m1 - m0);
+    // sum of S / 2^g, 2^g the power of two below N (rounded a lane at a time), then times 2^(g+1) / N = 2^g / H
+    const int sh = ie.ih;
+    int64_t sum = (hi << (32 - sh)) + (lo >> sh) + ((lo >> (sh - 1)) & 1);
+    for (int o = ln.L >> 1; o > 0; o >>= 1) sum += __shfl_xor_sync(FULLMASK, sum, o, ln.L);
+    const int64_t d0 = x[1];
+    __syncwarp();
+    pre += d0 - 2 * fx_mul(sum, inv);
+    const int P = sl * npairs + (t >> 1);
+    const int kx = fx_kx_out(kxs[2 * P + (t & 1)], growth ? fx_bits_of(scales, P) : 0);
+    for (int m = m0; m < m1; ++m) {
+      if (m > 0) pre += x[2 * m + 1];
+      x[2 * m + 1] = fx_out(md.alt_out ? -pre : pre, kx, p0, mul, inv);
     }
   }
 }
@@ -1623,11 +1832,7 @@ __device__ void op_dct(Ctx& c, const pgx_op& op, const pgx_instance& I) {
   const int c_tid = c.tid;
   const int n = c.slen[op.a];
   if (((n - 1) & 1) == 0 && n >= 3) {
-    // a tile with fewer line pairs per slot than warps (single instances, short passes) leaves
-    // warps idle in the warp-local form; there the CTA-wide form spreads each pair over all warps
-    // (per slot, so a multi-slot op and its one-op-per-slot split take the same form)
-    if ((op.k & PGX_DCT_CTA) || ((c_tb + 1) >> 1) < (c_nthreads >> 5)) op_dct_even_cta(c, op, I);
-    else op_dct_even(c, op, I);
+    op_dct_even(c, op, I.mat[op.mat]);
     return;
   }
   const int ns = nslot_of(op);  // paired-line path: one slot after the other
@@ -1660,17 +1865,18 @@ __device__ void dct_paired_slot(Ctx& c, int slot, const pgx_op& op, const pgx_in
   const int npairs = (c_tb + 1) >> 1;
   int nst = 0;
   for (int rem = L; rem > 1; rem /= next_radix(rem)) ++nst;
-  double2* bufs[2] = {c.f0, c.f1};
+  double2* const f0 = reinterpret_cast<double2*>(smem_dyn + c.f0);
+  double2* const f1 = reinterpret_cast<double2*>(smem_dyn + c.f1);
   int Ns = 1, rem = L, cur = 0;
   for (int s = 0; s < nst; ++s) {
     const int R = next_radix(rem);
-    const double2* src = bufs[cur];
-    double2* dst = bufs[cur ^ 1];
+    const double2* src = cur ? f1 : f0;
+    double2* dst = cur ? f0 : f1;
     if (s == 0) {
       if (nst == 1) {
-        stage_dispatch<true, false>(R, c, nullptr, c.f0, tw, L, Ns, npairs, x, ds);
+        stage_dispatch<true, false>(R, c, nullptr, f0, tw, L, Ns, npairs, x, ds);
       } else {
-        stage_dispatch<true, false>(R, c, nullptr, c.f0, tw, L, Ns, npairs, x, ds);
+        stage_dispatch<true, false>(R, c, nullptr, f0, tw, L, Ns, npairs, x, ds);
         cur = 0;
         Ns *= R;
         rem /= R;
@@ -1690,7 +1896,7 @@ __device__ void dct_paired_slot(Ctx& c, int slot, const pgx_op& op, const pgx_in
   if (nst == 1) {  // tiny transform: copy the single stage's output back
     for (int idx = c_tid; idx < c_tb * n; idx += c_nthreads) {
       int t = idx / n, k = idx - t * n;
-      double2 z = c.f0[(t >> 1) * c_fft_stride + k];
+      double2 z = f0[(t >> 1) * c_fft_stride + k];
       double y = (t & 1) ? z.y : z.x;
       if (ds.has_post) y *= ds.post(k, N);
       x[t * c_lcap + k] = y;
@@ -1700,8 +1906,9 @@ __device__ void dct_paired_slot(Ctx& c, int slot, const pgx_op& op, const pgx_in
 
 // ------------------------------------------------------------------ driver
 // One tile of one instance: the program's ops on shared-memory slots that start at `sm`.
+// `init`: bit s set if slot s has to start as zeros (pgx_init_mask).
 template <bool FFT, int KU>
-__device__ void run_program(const pgx_program& P, const pgx_instance& I, int tile, double* sm) {
+__device__ void run_program(const pgx_program& P, const pgx_instance& I, int tile, int sm, unsigned init) {
   Ctx c;
   c.tb = P.tb;
   c.lcap = P.lcap;
@@ -1711,24 +1918,26 @@ __device__ void run_program(const pgx_program& P, const pgx_instance& I, int til
   c.nlines = I.len[P.lines_len];
   const int nbuf = P.nslots + 1;
   c.sm = sm;
-  size_t off = (size_t)nbuf * c.tb * c.lcap;
+  const int off = nbuf * c.tb * c.lcap;
   c.fft_stride = pgx_fft_stride(P.fft_n);
   const int fs = pgx_fft_slots(P);
   const bool in_slot = FFT && pgx_fft_in_slot(P);
   const bool fft_in_spare = FFT && !in_slot && pgx_fft_in_spare(P);
-  const size_t fbuf = in_slot ? 0 : (size_t)fs * ((c.tb + 1) >> 1) * c.fft_stride;
-  double2* const f0 = reinterpret_cast<double2*>(c.sm + off + (off & 1));
-  double2* const f1 = fft_in_spare ? nullptr : f0 + fbuf;
-  c.ybuf = reinterpret_cast<double*>((fft_in_spare || in_slot ? f0 : f1) + fbuf);
+  const int fbuf = in_slot ? 0 : 2 * fs * ((c.tb + 1) >> 1) * c.fft_stride;
+  const int f0 = c.sm + off + (off & 1);
+  const int f1 = f0 + fbuf;
+  c.f0 = c.f1 = f0;
+  c.ybuf = (fft_in_spare || in_slot ? f0 : f1) + fbuf;
   const int fft_stride = c.fft_stride;
   for (int s = 0; s < nbuf; ++s) c.phys[s] = s;
   for (int s = 0; s < PGX_MAX_SLOTS; ++s) c.slen[s] = 0;
   c.spare = P.nslots;
   for (int s = 0; s < nbuf; ++s) {
-    double* b = c.sm + (size_t)s * c.tb * c.lcap;
+    if (!((init >> s) & 1)) continue;
+    double* b = smem_dyn + (c.sm + s * c.tb * c.lcap);
     for (int i = c.tid; i < c.tb * c.lcap; i += c.nthreads) b[i] = 0.0;
   }
-  __syncthreads();
+  if (init) __syncthreads();
   for (int o = 0; o < P.nops; ++o) {
     const pgx_op& op = P.ops[o];
     switch (op.code) {
@@ -1749,12 +1958,12 @@ __device__ void run_program(const pgx_program& P, const pgx_instance& I, int til
       case PGX_OP_DCT:
         if (FFT) {  // programs with DCT ops run the FFT kernels only
           if (op.k & PGX_DCT_SLOT) {  // ping-pong between the slot's own line pairs and the spare
-            c.f0 = reinterpret_cast<double2*>(slot_ptr(c, op.a));  // even tb: 16-byte aligned
-            c.f1 = reinterpret_cast<double2*>(spare_ptr(c));
-            c.fft_stride = c.lcap;  // a pair's two lines, in complex elements
+            c.f0 = c.sm + c.phys[op.a] * c.tb * c.lcap;
+            c.f1 = c.sm + c.spare * c.tb * c.lcap;
+            c.fft_stride = c.lcap;  // a pair's two lines
           } else {
-            c.f0 = in_slot ? nullptr : f0;
-            c.f1 = fft_in_spare ? reinterpret_cast<double2*>(spare_ptr(c)) : f1;
+            c.f0 = f0;
+            c.f1 = fft_in_spare ? c.sm + c.spare * c.tb * c.lcap : f1;
             c.fft_stride = in_slot ? 0 : fft_stride;
           }
           op_dct(c, op, I);
@@ -1778,8 +1987,7 @@ __device__ void run_program(const pgx_program& P, const pgx_instance& I, int til
 
 template <bool FFT, int KU>
 __device__ __forceinline__ void run_batched(const pgx_program& P, const pgx_instance* __restrict__ insts,
-                                            const int32_t* __restrict__ work) {
-  extern __shared__ __align__(16) double smem_dyn[];
+                                            const int32_t* __restrict__ work, unsigned init) {
   pgx_instance* sI = reinterpret_cast<pgx_instance*>(smem_dyn);
   const int inst = work[2 * blockIdx.x], tile = work[2 * blockIdx.x + 1];
   const int nwords = sizeof(pgx_instance) / 8;
@@ -1787,7 +1995,7 @@ __device__ __forceinline__ void run_batched(const pgx_program& P, const pgx_inst
   double* dst = reinterpret_cast<double*>(sI);
   for (int i = threadIdx.x; i < nwords; i += blockDim.x) dst[i] = src[i];
   __syncthreads();
-  run_program<FFT, KU>(P, *sI, tile, smem_dyn + (sizeof(pgx_instance) + 7) / 8);
+  run_program<FFT, KU>(P, *sI, tile, (int)((sizeof(pgx_instance) + 15) / 16 * 2), init);
 }
 
 // ------------------------------------------------------------- persistent steps
@@ -1804,11 +2012,9 @@ __global__ void __launch_bounds__(PGX_MAX_THREADS_FFT) line_program_persistent(
     const pgx_program* __restrict__ progs, int nprogs, const pgx_instance* __restrict__ descs, int ndescs,
     const pgx_persist_item* __restrict__ items, int nitems, int32_t* __restrict__ counters, int ncounters,
     int32_t* __restrict__ state, long long spin_limit) {
-  extern __shared__ __align__(16) double smem_dyn[];
   pgx_instance* sI = reinterpret_cast<pgx_instance*>(smem_dyn);
   pgx_program* sP = reinterpret_cast<pgx_program*>(reinterpret_cast<char*>(smem_dyn) +
                                                    ((sizeof(pgx_instance) + 15) / 16) * 16);
-  double* slots = smem_dyn + kPersistHead / 8;
   __shared__ int s_item, s_go;
   volatile int32_t* err = state + 1;
   // thread 0 holds the index of the CTA's next item: taken from the queue while the current item
@@ -1861,7 +2067,7 @@ __global__ void __launch_bounds__(PGX_MAX_THREADS_FFT) line_program_persistent(
       for (int i = threadIdx.x; i < words; i += blockDim.x) pd[i] = ps[i];
     }
     __syncthreads();
-    run_program<true, 4>(*sP, *sI, w.tile, slots);
+    run_program<true, 4>(*sP, *sI, w.tile, kPersistHead / 8, ~0u);
     // run_program ends every op with a block barrier: every store of the tile is done here
     if (threadIdx.x == 0) {
       __threadfence();
@@ -1873,26 +2079,24 @@ __global__ void __launch_bounds__(PGX_MAX_THREADS_FFT) line_program_persistent(
 // Two builds of the interpreter: with the FFT code (programs with DCT ops; up to 768 threads,
 // 80 registers a thread without spills) and without it (up to 1024 threads, 64 registers).
 __global__ void __launch_bounds__(PGX_MAX_THREADS) line_program_single(const __grid_constant__ pgx_program P,
-                                                                       const __grid_constant__ pgx_instance I) {
-  extern __shared__ __align__(16) double smem_dyn[];
-  run_program<false, 1>(P, I, blockIdx.x, smem_dyn);
+                                                                       const __grid_constant__ pgx_instance I, unsigned init) {
+  run_program<false, 1>(P, I, blockIdx.x, 0, init);
 }
 
 __global__ void __launch_bounds__(PGX_MAX_THREADS_FFT) line_program_single_fft(const __grid_constant__ pgx_program P,
-                                                                               const __grid_constant__ pgx_instance I) {
-  extern __shared__ __align__(16) double smem_dyn[];
-  run_program<true, 1>(P, I, blockIdx.x, smem_dyn);
+                                                                               const __grid_constant__ pgx_instance I, unsigned init) {
+  run_program<true, 1>(P, I, blockIdx.x, 0, init);
 }
 
 __global__ void __launch_bounds__(PGX_MAX_THREADS) line_program_batched(const __grid_constant__ pgx_program P,
                                                                         const pgx_instance* __restrict__ insts,
-                                                                        const int32_t* __restrict__ work) {
-  run_batched<false, 4>(P, insts, work);
+                                                                        const int32_t* __restrict__ work, unsigned init) {
+  run_batched<false, 4>(P, insts, work, init);
 }
 
 __global__ void __launch_bounds__(PGX_MAX_THREADS_FFT) line_program_batched_fft(
-    const __grid_constant__ pgx_program P, const pgx_instance* __restrict__ insts, const int32_t* __restrict__ work) {
-  run_batched<true, 4>(P, insts, work);
+    const __grid_constant__ pgx_program P, const pgx_instance* __restrict__ insts, const int32_t* __restrict__ work, unsigned init) {
+  run_batched<true, 4>(P, insts, work, init);
 }
 
 // The same builds for launches of fewer CTAs than the GPU has SMs (single instances): each CTA's
@@ -1900,13 +2104,13 @@ __global__ void __launch_bounds__(PGX_MAX_THREADS_FFT) line_program_batched_fft(
 // loads a thread cost there more than they hide.
 __global__ void __launch_bounds__(PGX_MAX_THREADS) line_program_batched_lat(const __grid_constant__ pgx_program P,
                                                                             const pgx_instance* __restrict__ insts,
-                                                                            const int32_t* __restrict__ work) {
-  run_batched<false, 1>(P, insts, work);
+                                                                            const int32_t* __restrict__ work, unsigned init) {
+  run_batched<false, 1>(P, insts, work, init);
 }
 
 __global__ void __launch_bounds__(PGX_MAX_THREADS_FFT) line_program_batched_fft_lat(
-    const __grid_constant__ pgx_program P, const pgx_instance* __restrict__ insts, const int32_t* __restrict__ work) {
-  run_batched<true, 1>(P, insts, work);
+    const __grid_constant__ pgx_program P, const pgx_instance* __restrict__ insts, const int32_t* __restrict__ work, unsigned init) {
+  run_batched<true, 1>(P, insts, work, init);
 }
 
 }  // namespace pgx
@@ -1960,13 +2164,14 @@ static int raise_smem_cap(const void* fn, int which) {
 int launch_single(const pgx_program* P, const pgx_instance* I, cudaStream_t s, int ntiles) {
   int64_t smem = pgx_program_smem(P);
   const bool fft = pgx_has_dct(*P);
+  const unsigned init = pgx_init_mask(*P);
   if (smem > 48 * 1024) {
     int e = fft ? raise_smem_cap((const void*)line_program_single_fft, 2)
                 : raise_smem_cap((const void*)line_program_single, 0);
     if (e) return e;
   }
-  if (fft) line_program_single_fft<<<ntiles, P->nthreads, smem, s>>>(*P, *I);
-  else line_program_single<<<ntiles, P->nthreads, smem, s>>>(*P, *I);
+  if (fft) line_program_single_fft<<<ntiles, P->nthreads, smem, s>>>(*P, *I, init);
+  else line_program_single<<<ntiles, P->nthreads, smem, s>>>(*P, *I, init);
   return (int)cudaGetLastError();
 }
 
@@ -2024,6 +2229,7 @@ int launch_batched(const pgx_program* P, const pgx_instance* d_insts, const int3
                    cudaStream_t s) {
   int64_t smem = pgx_program_smem(P) + ((sizeof(pgx_instance) + 15) / 16) * 16;
   const bool fft = pgx_has_dct(*P);
+  const unsigned init = pgx_init_mask(*P);
   const bool lat = nwork < sm_count();  // fewer CTAs than SMs: the latency build
   const void* fn = fft ? (lat ? (const void*)line_program_batched_fft_lat : (const void*)line_program_batched_fft)
                        : (lat ? (const void*)line_program_batched_lat : (const void*)line_program_batched);
@@ -2032,11 +2238,11 @@ int launch_batched(const pgx_program* P, const pgx_instance* d_insts, const int3
     if (e) return e;
   }
   if (fft) {
-    if (lat) line_program_batched_fft_lat<<<nwork, P->nthreads, smem, s>>>(*P, d_insts, d_work);
-    else line_program_batched_fft<<<nwork, P->nthreads, smem, s>>>(*P, d_insts, d_work);
+    if (lat) line_program_batched_fft_lat<<<nwork, P->nthreads, smem, s>>>(*P, d_insts, d_work, init);
+    else line_program_batched_fft<<<nwork, P->nthreads, smem, s>>>(*P, d_insts, d_work, init);
   } else {
-    if (lat) line_program_batched_lat<<<nwork, P->nthreads, smem, s>>>(*P, d_insts, d_work);
-    else line_program_batched<<<nwork, P->nthreads, smem, s>>>(*P, d_insts, d_work);
+    if (lat) line_program_batched_lat<<<nwork, P->nthreads, smem, s>>>(*P, d_insts, d_work, init);
+    else line_program_batched<<<nwork, P->nthreads, smem, s>>>(*P, d_insts, d_work, init);
   }
   return (int)cudaGetLastError();
 }

@@ -20,6 +20,7 @@
 #include <mutex>
 
 #include "pgx.h"
+#include "pgx_fixed.cuh"
 
 // Defined in pgx_api.cu: one DCT-I pass along an axis with a given table.
 int pgx_dct_pass(const double* in, int64_t in_s0, int64_t in_s1, int32_t n_in, double* out, int64_t out_s0,
@@ -29,8 +30,9 @@ bool pgx_fft_length_ok(int n);
 
 namespace {
 
-// complex entries per table: 2(n-1) twiddles and (n-1) / 2 for the n-1 fold coefficients, for every allowed n
-constexpr int kTwiddles = 3 * PGX_LMAX;
+// 16-byte entries per table: 2(n-1) twiddles, (n-1) / 2 for the n-1 fold coefficients, then (even n-1)
+// 2(n-1) fixed-point twiddles and one entry for 1 / (n-1), for every allowed n
+constexpr int kTwiddles = 5 * PGX_LMAX;
 
 static __device__ __align__(256) double g_noalloc_scratch[PGX_NOALLOC_SCRATCH_DOUBLES];
 static __device__ __align__(256) double2 g_noalloc_twiddles[2 * kTwiddles];
@@ -50,7 +52,13 @@ __global__ void noalloc_fill_twiddles(int L0, int L1) {
       s = q == 1 ? 1.0 : (q == 3 ? -1.0 : 0.0);
     }
     g_noalloc_twiddles[table * kTwiddles + k] = make_double2(c, -s);
-    if (k < L / 2) reinterpret_cast<double*>(g_noalloc_twiddles + table * kTwiddles + L)[k] = 0.5 + (-s);
+    const int N = L / 2;
+    if (k < N) reinterpret_cast<double*>(g_noalloc_twiddles + table * kTwiddles + L)[k] = 0.5 + (-s);
+    if ((N & 1) == 0) {
+      fx_tw* fx = reinterpret_cast<fx_tw*>(g_noalloc_twiddles + table * kTwiddles + L + N / 2);
+      fx[k] = fx_twiddle(k, N);
+      if (k == 0) fx[L] = fx_inverse(N);
+    }
   }
 }
 
