@@ -100,10 +100,126 @@ inline unsigned pgx_init_mask(const pgx_program& P) {
   return need;
 }
 
+// ---------------------------------------------------------------- lowering
+// What a launch runs: the program with neighbouring ops merged and without the barriers it does not need.
+// An op costs a CTA hundreds of cycles whatever it does, as much as a small tile's work in it (an empty one
+// ~410, ~69 instructions of a lone warp; reading the ops from shared memory or ahead of time, or comparing
+// codes instead of a jump table, changed nothing), and a barrier keeps neighbouring ops' loads apart.
+//   LOAD, STENCIL             one op that reads the array through the stencil
+//   [COPY] DIFF [SCALE]       one op: from another slot, with a factor
+//   a barrier after an op     only if an op up to the next barrier touches a buffer it writes, writes one it
+//                             reads, or both touch global memory and one of them writes it
+// Persistent launches take their programs from device memory as they are.
+namespace pgx {
+constexpr int kOpLoadStencil = 64, kOpDiffX = 65;  // codes of merged ops: in lowered programs only
+struct Lowered {
+  uint32_t init;       // slots that start as zeros (pgx_init_mask)
+  uint32_t nosync[3];  // ops without a barrier after them, a bit each
+  uint32_t merged;     // the program may hold merged ops
+  int16_t fft_slots, fft_in_slot, fft_in_spare;  // pgx_fft_slots, pgx_fft_in_slot, pgx_fft_in_spare
+  uint32_t mtb, mlcap;                           // multipliers of FastDiv for tb and lcap
+};
+}  // namespace pgx
+static_assert(PGX_MAX_OPS <= 96, "a barrier bit per op");
+
+inline void pgx_lower(const pgx_program& P, pgx_program& out, pgx::Lowered& how) {
+  using namespace pgx;
+  out = P;
+  how = Lowered{pgx_init_mask(P), {0, 0, 0}, 1, (int16_t)pgx_fft_slots(P), pgx_fft_in_slot(P), pgx_fft_in_spare(P),
+                0xffffffffu / (uint32_t)P.tb + 1u, 0xffffffffu / (uint32_t)P.lcap + 1u};
+  int n = 0;
+  for (int o = 0; o < P.nops; ++o) {
+    pgx_op op = P.ops[o];
+    if (op.code >= kOpLoadStencil) op.code = 0;  // no op of the ABI: does nothing, as before
+    const pgx_op* nx = o + 1 < P.nops ? &P.ops[o + 1] : nullptr;
+    if (op.code == PGX_OP_LOAD && op.par < 0 && op.alpha == 1.0 && nx && nx->code == PGX_OP_STENCIL && nx->a == op.a) {
+      op.code = kOpLoadStencil;
+      op.mat = nx->mat;
+      ++o;
+    } else {
+      int src = -1;
+      const pgx_op* d = nullptr;
+      if (op.code == PGX_OP_DIFF) {
+        d = &P.ops[o];
+      } else if (op.code == PGX_OP_COPY && op.par < 0 && op.alpha == 1.0 && op.a != op.b && nx && nx->code == PGX_OP_DIFF &&
+                 nx->a == op.a && nx->b <= 1 && nx->k == 1) {
+        src = op.b;
+        d = nx;
+      }
+      if (d && d->b <= 1 && d->k == 1) {
+        const int last = src >= 0 ? o + 1 : o;
+        const bool scale = last + 1 < P.nops && P.ops[last + 1].code == PGX_OP_SCALE && P.ops[last + 1].a == d->a;
+        if (src >= 0 || scale) {
+          pgx_op f = *d;
+          f.code = kOpDiffX;
+          f.arr = (int16_t)src;
+          f.alpha = scale ? P.ops[last + 1].alpha : 1.0;
+          f.par = scale ? P.ops[last + 1].par : (int16_t)-1;
+          op = f;
+          o = scale ? last + 1 : last;
+        }
+      }
+    }
+    out.ops[n++] = op;
+  }
+  out.nops = n;
+  // barriers: buffers as they move between the slots and the spare
+  int buf[PGX_MAX_SLOTS + 1];
+  for (int s = 0; s <= PGX_MAX_SLOTS; ++s) buf[s] = s;
+  int& spare = buf[P.nslots];
+  constexpr unsigned kGlobal = 1u << 30, kFft = 1u << 29;
+  unsigned rp = 0, wp = 0;  // read, written since the last barrier
+  for (int o = 0; o < n; ++o) {
+    const pgx_op& op = out.ops[o];
+    const unsigned a = 1u << buf[op.a], sp = 1u << spare;
+    unsigned r = 0, w = 0;
+    bool swap = false;
+    auto slots = [&]() {
+      unsigned m = 0;
+      for (int k = 0; k < (op.b > 1 ? op.b : 1) && op.a + k < P.nslots; ++k) m |= 1u << buf[op.a + k];
+      return m;
+    };
+    switch (op.code) {
+      case PGX_OP_LOAD: case kOpLoadStencil: w = a; r = kGlobal; break;
+      case PGX_OP_LOAD_ADD: case PGX_OP_LOAD_MUL: w = a; r = a | kGlobal; break;
+      case PGX_OP_STORE: case PGX_OP_STORE_ADD: r = a | kGlobal; w = kGlobal; break;
+      case PGX_OP_SCALE: r = w = a; break;
+      case PGX_OP_AXPY: case PGX_OP_MUL: case PGX_OP_COPY: r = a | (1u << buf[op.b]); w = a; break;
+      case PGX_OP_SETLEN: break;  // nothing, or between barriers of its own
+      case PGX_OP_STENCIL: case PGX_OP_STENCIL_T: case PGX_OP_BANDED: case PGX_OP_DENSE:
+        r = a;
+        w = sp;
+        swap = true;
+        break;
+      case PGX_OP_DIFF: case PGX_OP_DIFF_T: case PGX_OP_TDMA2: case PGX_OP_FDMA: case PGX_OP_FDMA_T:
+      case PGX_OP_POISSON: case PGX_OP_POISSON_T:
+        r = w = slots();
+        break;
+      case kOpDiffX: r = a | (op.arr >= 0 ? 1u << buf[op.arr] : 0u); w = a; break;
+      case PGX_OP_DCT: r = w = slots() | sp | kFft; break;
+      case PGX_OP_ZERO00: w = a; break;
+      default: r = w = ~0u; break;
+    }
+    if (o > 0) {
+      if ((wp & (r | w)) || (rp & w)) rp = wp = 0;
+      else how.nosync[(o - 1) >> 5] |= 1u << ((o - 1) & 31);
+    }
+    rp |= r;
+    wp |= w;
+    if (swap) {
+      const int t = buf[op.a];
+      buf[op.a] = spare;
+      spare = t;
+    }
+  }
+  if (n > 0) how.nosync[(n - 1) >> 5] |= 1u << ((n - 1) & 31);
+}
+
 namespace pgx {
 
-// 2k for k < PGX_LMAX: multipliers of the derivative recurrence, read through
-// the constant cache (lanes of a warp read the same k in lockstep).
+// 2k for k < PGX_LMAX: multipliers of the derivative recurrence.  In global memory: the lanes of a
+// warp read different ones, which the constant cache would serve one after the other (a derivative of
+// 65 points took 6,200 cycles of a CTA with them there, most of it that).
 struct TwoK {
   double v[PGX_LMAX];
 };
@@ -112,7 +228,7 @@ constexpr TwoK make_twok() {
   for (int i = 0; i < PGX_LMAX; ++i) t.v[i] = 2.0 * i;
   return t;
 }
-__constant__ TwoK c_twok = make_twok();
+__device__ const TwoK c_twok = make_twok();
 
 // x / d by a multiply-high for x < 2^18, d < 2^12 (offsets into a tile are below 2^15, lines and
 // chunks below 2^12): m = ceil(2^32 / d), exact while x (m d - 2^32) < 2^32.  A runtime division
@@ -130,6 +246,7 @@ __constant__ DivTable c_divs = make_divs();
 struct FastDiv {  // 1 <= d < PGX_LMAX + 16
   uint32_t d, m;
   __device__ __forceinline__ explicit FastDiv(int d_) : d((uint32_t)d_), m(c_divs.m[d_]) {}
+  __device__ __forceinline__ FastDiv(int d_, uint32_t m_) : d((uint32_t)d_), m(m_) {}
   __device__ __forceinline__ int div(int x) const { return d == 1 ? x : (int)__umulhi((uint32_t)x, m); }
 };
 
@@ -147,20 +264,33 @@ struct Ctx {
   int tb, lcap, nthreads, tid;
   int fft_stride;   // complex elements per pair in the FFT buffers
   int l0, nlines;   // first line of the tile, lines of the instance
-  int phys[PGX_MAX_SLOTS + 1];
-  int slen[PGX_MAX_SLOTS];
+  uint32_t mtb, mlcap;  // FastDiv multipliers of tb and lcap
   int spare;
+  // which buffer a slot is in (4 bits a slot) and the slots' lengths (16 bits): indexed by the op's
+  // fields, arrays would live in local memory, a load each
+  uint32_t physp;
+  uint64_t slens[2];
+  __device__ __forceinline__ int phys(int s) const { return (int)(physp >> (4 * s)) & 15; }
+  __device__ __forceinline__ int slen(int s) const {
+    return (int)((s < 4 ? slens[0] : slens[1]) >> (16 * (s & 3))) & 0xffff;
+  }
+  __device__ __forceinline__ void set_slen(int s, int n) {
+    const uint64_t m = 0xffffULL << (16 * (s & 3)), v = (uint64_t)n << (16 * (s & 3));
+    if (s < 4) slens[0] = (slens[0] & ~m) | v;
+    else slens[1] = (slens[1] & ~m) | v;
+  }
 };
+static_assert(PGX_MAX_SLOTS <= 8, "slot maps are packed for eight slots");
 
 __device__ __forceinline__ double* slot_ptr(const Ctx& c, int s) {
-  return smem_dyn + (c.sm + c.phys[s] * c.tb * c.lcap);
+  return smem_dyn + (c.sm + c.phys(s) * c.tb * c.lcap);
 }
 __device__ __forceinline__ double* spare_ptr(const Ctx& c) {
   return smem_dyn + (c.sm + c.spare * c.tb * c.lcap);
 }
 __device__ __forceinline__ void swap_spare(Ctx& c, int s) {
-  int t = c.phys[s];
-  c.phys[s] = c.spare;
+  const int t = c.phys(s);
+  c.physp = (c.physp & ~(15u << (4 * s))) | ((uint32_t)c.spare << (4 * s));
   c.spare = t;
 }
 
@@ -168,6 +298,11 @@ __device__ __forceinline__ double op_alpha(const pgx_op& op, const pgx_instance&
   if (op.par < 0) return op.alpha;
   const double p = I.par[op.par];
   return __double_as_longlong(op.alpha) == 0x3ff0000000000000LL ? p : op.alpha * p;
+}
+
+// Line of element idx of lines of n elements; a tile of one line (0 for any idx) needs no multiplier
+__device__ __forceinline__ FastDiv line_div(const Ctx& c, int n) {
+  return c.tb == 1 ? FastDiv(2, 0u) : FastDiv(max(n, 1));
 }
 
 // Whether alpha is 1, on its bits: a floating-point compare takes the FP64 pipe (66 cycles a warp),
@@ -199,7 +334,7 @@ __device__ void zero_tail(const Ctx& c, double* b, int from) {
   const int c_tid = c.tid;
   int w = c_lcap - from;
   if (w <= 0) return;
-  const FastDiv fw(w);
+  const FastDiv fw = line_div(c, w);
   for (int idx = c_tid; idx < c_tb * w; idx += c_nthreads) {
     const int t = fw.div(idx);
     b[t * c_lcap + from + idx - t * w] = 0.0;
@@ -217,9 +352,9 @@ __device__ __forceinline__ void load_loop(const Ctx& c, const View& v, double* s
   const int c_nthreads = c.nthreads;
   const int l0 = c.l0;
   const int nl = min(v.nl, c.nlines);
-  const bool contig = (v.se == 1);
+  const bool contig = v.se == 1 && c_tb > 1;
   const int total = c_tb * n;
-  const FastDiv fd(contig ? max(n, 1) : c_tb);
+  const FastDiv fd = contig ? FastDiv(max(n, 1)) : FastDiv(c_tb, c.mtb);
   // up to KU elements a thread per round, all their global loads issued before the first store to
   // the slot, so a round waits out one memory latency, not one an element (the build for
   // launches of fewer CTAs than SMs, KU = 1, keeps the shorter single-element loop)
@@ -255,8 +390,8 @@ __device__ void op_load(Ctx& c, const pgx_op& op, const pgx_instance& I, int axi
   const View v = view_of(I.arr[op.arr], axis);
   const double alpha = op_alpha(op, I);
   const bool one = is_one(alpha);
-  if (mode == 0) c.slen[op.a] = I.len[op.len];
-  const int n = c.slen[op.a];
+  if (mode == 0) c.set_slen(op.a, I.len[op.len]);
+  const int n = c.slen(op.a);
   double* s = slot_ptr(c, op.a);
   if (mode == 0) {
     if (one) load_loop<KU, true, 0>(c, v, s, n, alpha);
@@ -270,6 +405,54 @@ __device__ void op_load(Ctx& c, const pgx_op& op, const pgx_instance& I, int axi
   }
 }
 
+// LOAD and the STENCIL that follows it (pgx_lower): slot = S arr, read from the array twice (the second
+// time from L1) instead of through a slot, a barrier and the spare.
+template <int KU>
+__device__ void op_load_stencil(Ctx& c, const pgx_op& op, const pgx_instance& I, int axis) {
+  const View v = view_of(I.arr[op.arr], axis);
+  const double* sd = I.mat[op.mat];
+  const int M = I.len[op.len], N = min(M + 2, c.lcap);
+  c.set_slen(op.a, M + 2);
+  double* s = slot_ptr(c, op.a);
+  const int c_tb = c.tb;
+  const int c_lcap = c.lcap;
+  const int c_nthreads = c.nthreads;
+  const int l0 = c.l0;
+  const int nl = min(v.nl, c.nlines), ne = min(v.ne, M);
+  const bool contig = v.se == 1 && c_tb > 1;
+  const int total = c_tb * N;
+  const FastDiv fd = contig ? FastDiv(N) : FastDiv(c_tb, c.mtb);
+  for (int base = c.tid; base < total; base += KU * c_nthreads) {
+    double x[KU], y[KU], w[KU];
+    int off[KU];
+#pragma unroll
+    for (int u = 0; u < KU; ++u) {
+      const int idx = base + u * c_nthreads;
+      x[u] = y[u] = w[u] = 0.0;
+      off[u] = -1;
+      if (idx < total) {
+        int t, i;
+        if (contig) { t = fd.div(idx); i = idx - t * N; }
+        else { i = fd.div(idx); t = idx - i * c_tb; }
+        const int line = l0 + t;
+        off[u] = t * c_lcap + i;
+        if (line < nl) {
+          const double* p = v.p + (int64_t)line * v.sl;
+          if (i < ne) x[u] = p[(int64_t)i * v.se];
+          if (i >= 2) {
+            w[u] = __ldg(sd + i - 2);
+            if (i - 2 < ne) y[u] = p[(int64_t)(i - 2) * v.se];
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < KU; ++u)
+      if (off[u] >= 0) s[off[u]] = fma(w[u], y[u], x[u]);
+  }
+  zero_tail(c, s, N);
+}
+
 template <int KU, bool ONE, bool ADD>
 __device__ __forceinline__ void store_loop(const Ctx& c, const View& v, const double* s, double alpha) {
   const int c_tb = c.tb;
@@ -278,9 +461,9 @@ __device__ __forceinline__ void store_loop(const Ctx& c, const View& v, const do
   const int l0 = c.l0;
   const int nl = min(v.nl, c.nlines);
   const int n = v.ne;
-  const bool contig = (v.se == 1);
+  const bool contig = v.se == 1 && c_tb > 1;
   const int total = c_tb * n;
-  const FastDiv fd(contig ? max(n, 1) : c_tb);
+  const FastDiv fd = contig ? FastDiv(max(n, 1)) : FastDiv(c_tb, c.mtb);
   // up to KU elements a thread per round, every load (the slot's and, to accumulate, the array's)
   // before the first store: one memory latency per round, not per element
   for (int base = c.tid; base < total; base += KU * c_nthreads) {
@@ -335,14 +518,14 @@ __device__ void op_pointwise(Ctx& c, const pgx_op& op, const pgx_instance& I) {
   const bool one = is_one(alpha);
   double* a = slot_ptr(c, op.a);
   const double* b = op.b >= 0 ? slot_ptr(c, op.b) : nullptr;
-  int n = c.slen[op.a];
+  int n = c.slen(op.a);
   if (op.code != PGX_OP_SCALE) {
-    int nb = c.slen[op.b];
+    int nb = c.slen(op.b);
     if (op.code == PGX_OP_COPY) n = nb;
     else if (nb > n) n = nb;
-    c.slen[op.a] = n;
+    c.set_slen(op.a, n);
   }
-  const FastDiv fn(n > 0 ? n : 1);
+  const FastDiv fn = line_div(c, n);
   for (int idx = c_tid; idx < c_tb * n; idx += c_nthreads) {
     const int t = fn.div(idx);
     const int o = t * c_lcap + idx - t * n;
@@ -363,9 +546,13 @@ __device__ void op_pointwise(Ctx& c, const pgx_op& op, const pgx_instance& I) {
 
 __device__ void op_setlen(Ctx& c, const pgx_op& op, const pgx_instance& I) {
   int n = I.len[op.len];
-  int old = c.slen[op.a];
-  if (n < old) zero_tail(c, slot_ptr(c, op.a), n);
-  c.slen[op.a] = n;
+  int old = c.slen(op.a);
+  if (n < old) {  // no barrier follows a SETLEN (pgx_lower): one that touches the line brings its own
+    __syncthreads();
+    zero_tail(c, slot_ptr(c, op.a), n);
+    __syncthreads();
+  }
+  c.set_slen(op.a, n);
 }
 
 // ------------------------------------------------------------------ stencils
@@ -379,9 +566,9 @@ __device__ void op_stencil(Ctx& c, const pgx_op& op, const pgx_instance& I) {
   const double* sd = I.mat[op.mat];
   const double* x = slot_ptr(c, op.a);
   double* y = spare_ptr(c);
-  const int M = c.slen[op.a], N = M + 2;
+  const int M = c.slen(op.a), N = M + 2;
   const int total = c_tb * c_lcap;
-  const FastDiv fl(c_lcap);
+  const FastDiv fl(c_lcap, c.mlcap);
   constexpr int kU = KU;  // the table loads of kU elements before their stores
   for (int base = c_tid; base < total; base += kU * c_nthreads) {
     double r[kU];
@@ -403,7 +590,7 @@ __device__ void op_stencil(Ctx& c, const pgx_op& op, const pgx_instance& I) {
       if (base + u * c_nthreads < total) y[base + u * c_nthreads] = r[u];
   }
   swap_spare(c, op.a);
-  c.slen[op.a] = N;
+  c.set_slen(op.a, N);
 }
 
 // (S^T u)_i = u_i + s_i u_{i+2},  i < N-2.
@@ -416,9 +603,9 @@ __device__ void op_stencil_t(Ctx& c, const pgx_op& op, const pgx_instance& I) {
   const double* sd = I.mat[op.mat];
   const double* x = slot_ptr(c, op.a);
   double* y = spare_ptr(c);
-  const int N = c.slen[op.a], M = N - 2;
+  const int N = c.slen(op.a), M = N - 2;
   const int total = c_tb * c_lcap;
-  const FastDiv fl(c_lcap);
+  const FastDiv fl(c_lcap, c.mlcap);
   constexpr int kU = KU;  // the table loads of kU elements before their stores
   for (int base = c_tid; base < total; base += kU * c_nthreads) {
     double r[kU];
@@ -439,7 +626,7 @@ __device__ void op_stencil_t(Ctx& c, const pgx_op& op, const pgx_instance& I) {
       if (base + u * c_nthreads < total) y[base + u * c_nthreads] = r[u];
   }
   swap_spare(c, op.a);
-  c.slen[op.a] = M;
+  c.set_slen(op.a, M);
 }
 
 // ------------------------------------------------ sequential parity chains
@@ -602,7 +789,7 @@ __device__ void op_tdma2(Ctx& c, const pgx_op& op, const pgx_instance& I) {
       const int r = w - s * 2 * c_tb;
       p = r / c_tb;
       t = r - p * c_tb;
-      const int n = c.slen[op.a + s];
+      const int n = c.slen(op.a + s);
       if (p >= n) continue;
       tdma_chain_warp(slot_ptr(c, op.a + s) + t * c_lcap, I.mat[op.mat], n, p, lane);
     }
@@ -612,7 +799,7 @@ __device__ void op_tdma2(Ctx& c, const pgx_op& op, const pgx_instance& I) {
     Ctx cc = c;
     cc.tid = c_tid + base;
     if (!chain_of(cc, ns, s, t, p)) continue;
-    const int n = c.slen[op.a + s];
+    const int n = c.slen(op.a + s);
     if (p >= n) continue;
     const double* tab = I.mat[op.mat];
     double* x = slot_ptr(c, op.a + s) + t * c_lcap;
@@ -662,25 +849,35 @@ __device__ __forceinline__ LineLanes line_lanes(const Ctx& c, int nl) {
   return g;
 }
 
-__device__ void op_diff(Ctx& c, const pgx_op& op) {
+// Each lane's chunk starts at an even index, so the two parity classes have fixed places in the loops.
+// `src`: slot the coefficients come from (op.a itself, or with one slot another one); alpha: a factor
+// on the result (a SCALE that follows, see pgx_lower).
+__device__ void op_diff(Ctx& c, const pgx_op& op, int src, double alpha) {
   const int c_tb = c.tb;
   const int c_lcap = c.lcap;
   const int ns = nslot_of(op);
+  const bool one = is_one(alpha);
+  if (src != op.a) c.set_slen(op.a, c.slen(src));
   const LineLanes g = line_lanes(c, ns * c_tb);
+  const FastDiv ft(c_tb, c.mtb);
+  const int lg = __ffs(g.L) - 1;
   for (int base = g.first; base < g.nl; base += g.stride) {  // the same trip count for the whole warp
     const int w = base + g.grp;
     const bool valid = w < g.nl;
-    const int s = valid ? w / c_tb : 0, t = valid ? w - s * c_tb : 0;
-    const int n = valid ? c.slen[op.a + s] : 0;
+    const int s = valid ? ft.div(w) : 0, t = valid ? w - s * c_tb : 0;
+    const int n = valid ? c.slen(op.a + s) : 0;
     double* x = slot_ptr(c, op.a + s) + t * c_lcap;
-    const int chunk = (n + g.L - 1) / g.L;
+    const double* y = src != op.a ? slot_ptr(c, src) + t * c_lcap : x;
+    const int chunk = 2 * ((((n + 1) >> 1) + g.L - 1) >> lg);
     const int a = min(g.sub * chunk, n), b = min(a + chunk, n);
     for (int rep = 0; rep < op.k; ++rep) {
-      double tot[2] = {0.0, 0.0};
-      for (int i = a; i < b; ++i) tot[i & 1] = fma(c_twok.v[i], x[i], tot[i & 1]);
-      const double c1 = valid ? x[1] : 0.0;
+      double t0 = 0.0, t1 = 0.0;  // sums of 2k c_k over the chunk's even and odd k
+      for (int i = a; i < b; i += 2) {
+        t0 = fma(__ldg(c_twok.v + i), y[i], t0);
+        if (i + 1 < b) t1 = fma(__ldg(c_twok.v + i + 1), y[i + 1], t1);
+      }
       // exclusive suffix sums of the chunk totals over the lanes above this one (of this line)
-      double in0 = tot[0], in1 = tot[1];
+      double in0 = t0, in1 = t1;
       for (int o = 1; o < g.L; o <<= 1) {
         const double v0 = __shfl_down_sync(0xffffffffu, in0, o, g.L);
         const double v1 = __shfl_down_sync(0xffffffffu, in1, o, g.L);
@@ -689,41 +886,53 @@ __device__ void op_diff(Ctx& c, const pgx_op& op) {
           in1 += v1;
         }
       }
-      double acc[2] = {in0 - tot[0], in1 - tot[1]};  // S_p(b)
-      __syncwarp();
-      for (int i = b - 1; i >= a; --i) {
-        const double wi = c_twok.v[i] * x[i];
-        x[i] = acc[(i + 1) & 1];  // dc_i = S_{(i+1) mod 2}(i+1)
-        acc[i & 1] += wi;
+      double s0 = __shfl_down_sync(0xffffffffu, in0, 1, g.L);
+      double s1 = __shfl_down_sync(0xffffffffu, in1, 1, g.L);
+      if (g.sub == g.L - 1) s0 = s1 = 0.0;
+      for (int i = ((b - a + 1) >> 1) * 2 + a - 2; i >= a; i -= 2) {
+        const double e = y[i];
+        if (i + 1 < b) {
+          const double d = y[i + 1];
+          x[i + 1] = one ? s0 : alpha * s0;  // dc_i = S_{(i+1) mod 2}(i+1)
+          s1 = fma(__ldg(c_twok.v + i + 1), d, s1);
+        }
+        double r = i > 0 ? s1 : pgx_half_signed(s1, false);
+        if (!one) r *= alpha;
+        x[i] = r;
+        s0 = fma(__ldg(c_twok.v + i), e, s0);
       }
-      __syncwarp();
-      if (valid && g.sub == 0) x[0] = fma(0.5, n > 2 ? x[2] : 0.0, c1);
       __syncwarp();
     }
   }
+  if (src != op.a) zero_tail(c, slot_ptr(c, op.a), c.slen(op.a));
 }
 
 // Transpose of the derivative recurrence (adjoint of op_diff), in place:
 //   (D^T y)_i = 2i sum_{1 <= j < i, j = i+1 mod 2} y_j + y_0 [i odd] (1 if i = 1 else i).
-// Forward prefix sums per parity class, L lanes a line.
+// Forward prefix sums per parity class, L lanes a line, chunks from even indices.
 __device__ void op_diff_t(Ctx& c, const pgx_op& op) {
   const int c_tb = c.tb;
   const int c_lcap = c.lcap;
   const int ns = nslot_of(op);
   const LineLanes g = line_lanes(c, ns * c_tb);
+  const FastDiv ft(c_tb, c.mtb);
+  const int lg = __ffs(g.L) - 1;
   for (int base = g.first; base < g.nl; base += g.stride) {
     const int w = base + g.grp;
     const bool valid = w < g.nl;
-    const int s = valid ? w / c_tb : 0, t = valid ? w - s * c_tb : 0;
-    const int n = valid ? c.slen[op.a + s] : 0;
+    const int s = valid ? ft.div(w) : 0, t = valid ? w - s * c_tb : 0;
+    const int n = valid ? c.slen(op.a + s) : 0;
     double* x = slot_ptr(c, op.a + s) + t * c_lcap;
-    const int chunk = (n + g.L - 1) / g.L;
+    const int chunk = 2 * ((((n + 1) >> 1) + g.L - 1) >> lg);
     const int a = min(g.sub * chunk, n), b = min(a + chunk, n);
     for (int rep = 0; rep < op.k; ++rep) {
-      double tot[2] = {0.0, 0.0};
-      for (int i = max(a, 1); i < b; ++i) tot[i & 1] += x[i];
+      double t0 = 0.0, t1 = 0.0;  // sums over the chunk's even and odd j >= 1
+      for (int i = a; i < b; i += 2) {
+        if (i > 0) t0 += x[i];
+        if (i + 1 < b) t1 += x[i + 1];
+      }
       const double y0 = valid ? x[0] : 0.0;
-      double in0 = tot[0], in1 = tot[1];
+      double in0 = t0, in1 = t1;
       for (int o = 1; o < g.L; o <<= 1) {
         const double v0 = __shfl_up_sync(0xffffffffu, in0, o, g.L);
         const double v1 = __shfl_up_sync(0xffffffffu, in1, o, g.L);
@@ -732,14 +941,18 @@ __device__ void op_diff_t(Ctx& c, const pgx_op& op) {
           in1 += v1;
         }
       }
-      double acc[2] = {in0 - tot[0], in1 - tot[1]};  // sums over j < a, j >= 1
-      __syncwarp();
-      for (int i = a; i < b; ++i) {
-        const double yi = x[i];
-        double v = c_twok.v[i] * acc[(i + 1) & 1];
-        if (i & 1) v = fma(i == 1 ? 1.0 : 0.5 * c_twok.v[i], y0, v);
-        x[i] = v;
-        if (i >= 1) acc[i & 1] += yi;
+      double s0 = __shfl_up_sync(0xffffffffu, in0, 1, g.L);  // sums over j < a, j >= 1
+      double s1 = __shfl_up_sync(0xffffffffu, in1, 1, g.L);
+      if (g.sub == 0) s0 = s1 = 0.0;
+      for (int i = a; i < b; i += 2) {
+        const double e = x[i];
+        x[i] = __ldg(c_twok.v + i) * s1;
+        if (i > 0) s0 += e;
+        if (i + 1 < b) {
+          const double d = x[i + 1], w1 = __ldg(c_twok.v + i + 1);
+          x[i + 1] = fma(i == 0 ? 1.0 : pgx_half_signed(w1, false), y0, w1 * s0);
+          s1 += d;
+        }
       }
       __syncwarp();
     }
@@ -833,7 +1046,7 @@ __device__ void op_fdma(Ctx& c, const pgx_op& op, const pgx_instance& I, bool pe
       const int r = w - s * 2 * c_tb;
       p = r / c_tb;
       t = r - p * c_tb;
-      const int n = c.slen[op.a + s];
+      const int n = c.slen(op.a + s);
       const int line = c_l0 + t;
       if (p >= n || line >= c_nlines) continue;
       const double* tab = I.mat[op.mat + (per_line ? 0 : s)];
@@ -848,7 +1061,7 @@ __device__ void op_fdma(Ctx& c, const pgx_op& op, const pgx_instance& I, bool pe
     Ctx cc = c;
     cc.tid = c_tid + base;
     if (!chain_of(cc, ns, s, t, p)) continue;
-    const int n = c.slen[op.a + s];
+    const int n = c.slen(op.a + s);
     const int line = c_l0 + t;
     if (p >= n || line >= c_nlines) continue;
     const double* tab = I.mat[op.mat + (per_line ? 0 : s)];
@@ -868,11 +1081,11 @@ __device__ void op_banded(Ctx& c, const pgx_op& op, const pgx_instance& I) {
   const double* A = I.mat[op.mat];
   const int rows = I.len[op.len];
   const int nd = op.k, off0 = op.b;
-  const int cols = c.slen[op.a];
+  const int cols = c.slen(op.a);
   const double* x = slot_ptr(c, op.a);
   double* y = spare_ptr(c);
   const int total = c_tb * c_lcap;
-  const FastDiv fl(c_lcap);
+  const FastDiv fl(c_lcap, c.mlcap);
   constexpr int kU = KU > 2 ? 2 : KU;  // the matrix loads of kU rows before their stores
   for (int base = c_tid; base < total; base += kU * c_nthreads) {
     double acc[kU];
@@ -896,7 +1109,7 @@ __device__ void op_banded(Ctx& c, const pgx_op& op, const pgx_instance& I) {
       if (base + u * c_nthreads < total) y[base + u * c_nthreads] = acc[u];
   }
   swap_spare(c, op.a);
-  c.slen[op.a] = rows;
+  c.set_slen(op.a, rows);
 }
 
 // D (8x8) += A (8x4, row-major) B (4x8, column-major) on the FP64 tensor cores; per lane
@@ -916,7 +1129,7 @@ __device__ void op_dense_mma(Ctx& c, const pgx_op& op, const pgx_instance& I) {
   const int c_tid = c.tid;
   const double* A = I.mat[op.mat];
   const int rows = I.len[op.len];
-  const int cols = c.slen[op.a];
+  const int cols = c.slen(op.a);
   const double* x = slot_ptr(c, op.a);
   double* y = spare_ptr(c);
   zero_tail(c, y, rows);
@@ -950,7 +1163,7 @@ __device__ void op_dense_mma(Ctx& c, const pgx_op& op, const pgx_instance& I) {
   }
   __syncthreads();
   swap_spare(c, op.a);
-  c.slen[op.a] = rows;
+  c.set_slen(op.a, rows);
 }
 
 __device__ void op_dense(Ctx& c, const pgx_op& op, const pgx_instance& I) {
@@ -964,11 +1177,11 @@ __device__ void op_dense(Ctx& c, const pgx_op& op, const pgx_instance& I) {
   }
   const double* A = I.mat[op.mat];
   const int rows = I.len[op.len];
-  const int cols = c.slen[op.a];
+  const int cols = c.slen(op.a);
   const double* x = slot_ptr(c, op.a);
   double* y = spare_ptr(c);
   zero_tail(c, y, rows);
-  const FastDiv ft(c_tb);
+  const FastDiv ft(c_tb, c.mtb);
   for (int idx = c_tid; idx < c_tb * rows; idx += c_nthreads) {
     const int r = ft.div(idx), t = idx - r * c_tb;
     const double* xl = x + t * c_lcap;
@@ -986,7 +1199,7 @@ __device__ void op_dense(Ctx& c, const pgx_op& op, const pgx_instance& I) {
   }
   __syncthreads();
   swap_spare(c, op.a);
-  c.slen[op.a] = rows;
+  c.set_slen(op.a, rows);
 }
 
 // ---------------------------------------------------------------- DCT-I
@@ -1233,7 +1446,7 @@ struct FxSlots {
 };
 __device__ __forceinline__ int64_t* fx_sm(int off) { return reinterpret_cast<int64_t*>(smem_dyn) + off; }
 __device__ __forceinline__ int64_t* fx_line(const Ctx& c, int slot, int t) {
-  return fx_sm(c.sm + (c.phys[slot] * c.tb + t) * c.lcap);
+  return fx_sm(c.sm + (c.phys(slot) * c.tb + t) * c.lcap);
 }
 __device__ __forceinline__ int64_t* fx_pair(const FxSlots& m, const FxBuf& b, int P) {
   if (m.npairs < 0) return fx_sm(b.p + P * b.pair);
@@ -1604,7 +1817,7 @@ __device__ __forceinline__ void op_dct_even(Ctx& c, const pgx_op& op, const doub
   const int ns = nslot_of(op);
   const int npairs = (tb + 1) >> 1;
   const int nall = ns * npairs;  // line pairs of all slots; pair P = s * npairs + pr
-  const int n = c.slen[slot0];
+  const int n = c.slen(slot0);
   const int N = n - 1, H = N / 2;
   const FxMode md = fx_mode(op.k & PGX_DCT_MODE_MASK);
   const bool in_slot = (op.k & PGX_DCT_SLOT) != 0;
@@ -1716,7 +1929,7 @@ __device__ __forceinline__ void op_dct_even(Ctx& c, const pgx_op& op, const doub
   fx_sync(g.cta);
   // FFT of length N over the pairs
   const FxSlots ms = {&c, slot0, ns == 1 || odd_tile ? -1 : npairs};
-  const FxBuf src = odd_tile ? b0 : FxBuf{c.sm + c.phys[slot0] * tb * lcap, lcap, 2 * lcap};
+  const FxBuf src = odd_tile ? b0 : FxBuf{c.sm + c.phys(slot0) * tb * lcap, lcap, 2 * lcap};
   int zp;
   switch (N) {
     case 16: zp = fx_fft_n<16>(ms, g, src, b0, b1, tw, scales); break;
@@ -1830,7 +2043,7 @@ __device__ void op_dct(Ctx& c, const pgx_op& op, const pgx_instance& I) {
   const int c_tb = c.tb;
   const int c_nthreads = c.nthreads;
   const int c_tid = c.tid;
-  const int n = c.slen[op.a];
+  const int n = c.slen(op.a);
   if (((n - 1) & 1) == 0 && n >= 3) {
     op_dct_even(c, op, I.mat[op.mat]);
     return;
@@ -1853,7 +2066,7 @@ __device__ void dct_paired_slot(Ctx& c, int slot, const pgx_op& op, const pgx_in
   const int c_nthreads = c.nthreads;
   const int c_tid = c.tid;
   const int c_fft_stride = c.fft_stride;
-  const int n = c.slen[slot];
+  const int n = c.slen(slot);
   if (2 * (n - 1) > c_fft_stride) {  // buffer sized for a shorter even length: refuse loudly
     for (int idx = c_tid; idx < c_tb * n; idx += c_nthreads) x_nan(c, slot, idx, n);
     return;
@@ -1906,9 +2119,8 @@ __device__ void dct_paired_slot(Ctx& c, int slot, const pgx_op& op, const pgx_in
 
 // ------------------------------------------------------------------ driver
 // One tile of one instance: the program's ops on shared-memory slots that start at `sm`.
-// `init`: bit s set if slot s has to start as zeros (pgx_init_mask).
 template <bool FFT, int KU>
-__device__ void run_program(const pgx_program& P, const pgx_instance& I, int tile, int sm, unsigned init) {
+__device__ void run_program(const pgx_program& P, const pgx_instance& I, int tile, int sm, const Lowered& how) {
   Ctx c;
   c.tb = P.tb;
   c.lcap = P.lcap;
@@ -1916,28 +2128,29 @@ __device__ void run_program(const pgx_program& P, const pgx_instance& I, int til
   c.tid = threadIdx.x;
   c.l0 = tile * P.tb;
   c.nlines = I.len[P.lines_len];
+  c.mtb = how.mtb;
+  c.mlcap = how.mlcap;
   const int nbuf = P.nslots + 1;
   c.sm = sm;
   const int off = nbuf * c.tb * c.lcap;
   c.fft_stride = pgx_fft_stride(P.fft_n);
-  const int fs = pgx_fft_slots(P);
-  const bool in_slot = FFT && pgx_fft_in_slot(P);
-  const bool fft_in_spare = FFT && !in_slot && pgx_fft_in_spare(P);
-  const int fbuf = in_slot ? 0 : 2 * fs * ((c.tb + 1) >> 1) * c.fft_stride;
+  const bool in_slot = FFT && how.fft_in_slot;
+  const bool fft_in_spare = FFT && !in_slot && how.fft_in_spare;
+  const int fbuf = in_slot ? 0 : 2 * how.fft_slots * ((c.tb + 1) >> 1) * c.fft_stride;
   const int f0 = c.sm + off + (off & 1);
   const int f1 = f0 + fbuf;
   c.f0 = c.f1 = f0;
   c.ybuf = (fft_in_spare || in_slot ? f0 : f1) + fbuf;
   const int fft_stride = c.fft_stride;
-  for (int s = 0; s < nbuf; ++s) c.phys[s] = s;
-  for (int s = 0; s < PGX_MAX_SLOTS; ++s) c.slen[s] = 0;
+  c.physp = 0x76543210u;
+  c.slens[0] = c.slens[1] = 0;
   c.spare = P.nslots;
   for (int s = 0; s < nbuf; ++s) {
-    if (!((init >> s) & 1)) continue;
+    if (!((how.init >> s) & 1)) continue;
     double* b = smem_dyn + (c.sm + s * c.tb * c.lcap);
     for (int i = c.tid; i < c.tb * c.lcap; i += c.nthreads) b[i] = 0.0;
   }
-  if (init) __syncthreads();
+  if (how.init) __syncthreads();
   for (int o = 0; o < P.nops; ++o) {
     const pgx_op& op = P.ops[o];
     switch (op.code) {
@@ -1954,11 +2167,17 @@ __device__ void run_program(const pgx_program& P, const pgx_instance& I, int til
       case PGX_OP_STENCIL: op_stencil<KU>(c, op, I); break;
       case PGX_OP_STENCIL_T: op_stencil_t<KU>(c, op, I); break;
       case PGX_OP_TDMA2: op_tdma2(c, op, I); break;
-      case PGX_OP_DIFF: op_diff(c, op); break;
+      case PGX_OP_DIFF: op_diff(c, op, op.a, 1.0); break;
+      case kOpDiffX:
+        if (how.merged) op_diff(c, op, op.arr >= 0 ? op.arr : op.a, op_alpha(op, I));
+        break;
+      case kOpLoadStencil:
+        if (how.merged) op_load_stencil<KU>(c, op, I, P.axis);
+        break;
       case PGX_OP_DCT:
         if (FFT) {  // programs with DCT ops run the FFT kernels only
           if (op.k & PGX_DCT_SLOT) {  // ping-pong between the slot's own line pairs and the spare
-            c.f0 = c.sm + c.phys[op.a] * c.tb * c.lcap;
+            c.f0 = c.sm + c.phys(op.a) * c.tb * c.lcap;
             c.f1 = c.sm + c.spare * c.tb * c.lcap;
             c.fft_stride = c.lcap;  // a pair's two lines
           } else {
@@ -1981,13 +2200,13 @@ __device__ void run_program(const pgx_program& P, const pgx_instance& I, int til
         break;
       default: break;
     }
-    __syncthreads();
+    if (!((how.nosync[o >> 5] >> (o & 31)) & 1)) __syncthreads();
   }
 }
 
 template <bool FFT, int KU>
 __device__ __forceinline__ void run_batched(const pgx_program& P, const pgx_instance* __restrict__ insts,
-                                            const int32_t* __restrict__ work, unsigned init) {
+                                            const int32_t* __restrict__ work, const Lowered& how) {
   pgx_instance* sI = reinterpret_cast<pgx_instance*>(smem_dyn);
   const int inst = work[2 * blockIdx.x], tile = work[2 * blockIdx.x + 1];
   const int nwords = sizeof(pgx_instance) / 8;
@@ -1995,7 +2214,7 @@ __device__ __forceinline__ void run_batched(const pgx_program& P, const pgx_inst
   double* dst = reinterpret_cast<double*>(sI);
   for (int i = threadIdx.x; i < nwords; i += blockDim.x) dst[i] = src[i];
   __syncthreads();
-  run_program<FFT, KU>(P, *sI, tile, (int)((sizeof(pgx_instance) + 15) / 16 * 2), init);
+  run_program<FFT, KU>(P, *sI, tile, (int)((sizeof(pgx_instance) + 15) / 16 * 2), how);
 }
 
 // ------------------------------------------------------------- persistent steps
@@ -2067,7 +2286,9 @@ __global__ void __launch_bounds__(PGX_MAX_THREADS_FFT) line_program_persistent(
       for (int i = threadIdx.x; i < words; i += blockDim.x) pd[i] = ps[i];
     }
     __syncthreads();
-    run_program<true, 4>(*sP, *sI, w.tile, kPersistHead / 8, ~0u);
+    run_program<true, 4>(*sP, *sI, w.tile, kPersistHead / 8,
+                         Lowered{~0u, {0, 0, 0}, 0, (int16_t)pgx_fft_slots(*sP), pgx_fft_in_slot(*sP),
+                                 pgx_fft_in_spare(*sP), c_divs.m[sP->tb], c_divs.m[sP->lcap]});
     // run_program ends every op with a block barrier: every store of the tile is done here
     if (threadIdx.x == 0) {
       __threadfence();
@@ -2079,24 +2300,24 @@ __global__ void __launch_bounds__(PGX_MAX_THREADS_FFT) line_program_persistent(
 // Two builds of the interpreter: with the FFT code (programs with DCT ops; up to 768 threads,
 // 80 registers a thread without spills) and without it (up to 1024 threads, 64 registers).
 __global__ void __launch_bounds__(PGX_MAX_THREADS) line_program_single(const __grid_constant__ pgx_program P,
-                                                                       const __grid_constant__ pgx_instance I, unsigned init) {
-  run_program<false, 1>(P, I, blockIdx.x, 0, init);
+                                                                       const __grid_constant__ pgx_instance I, const __grid_constant__ Lowered how) {
+  run_program<false, 1>(P, I, blockIdx.x, 0, how);
 }
 
 __global__ void __launch_bounds__(PGX_MAX_THREADS_FFT) line_program_single_fft(const __grid_constant__ pgx_program P,
-                                                                               const __grid_constant__ pgx_instance I, unsigned init) {
-  run_program<true, 1>(P, I, blockIdx.x, 0, init);
+                                                                               const __grid_constant__ pgx_instance I, const __grid_constant__ Lowered how) {
+  run_program<true, 1>(P, I, blockIdx.x, 0, how);
 }
 
 __global__ void __launch_bounds__(PGX_MAX_THREADS) line_program_batched(const __grid_constant__ pgx_program P,
                                                                         const pgx_instance* __restrict__ insts,
-                                                                        const int32_t* __restrict__ work, unsigned init) {
-  run_batched<false, 4>(P, insts, work, init);
+                                                                        const int32_t* __restrict__ work, const __grid_constant__ Lowered how) {
+  run_batched<false, 4>(P, insts, work, how);
 }
 
 __global__ void __launch_bounds__(PGX_MAX_THREADS_FFT) line_program_batched_fft(
-    const __grid_constant__ pgx_program P, const pgx_instance* __restrict__ insts, const int32_t* __restrict__ work, unsigned init) {
-  run_batched<true, 4>(P, insts, work, init);
+    const __grid_constant__ pgx_program P, const pgx_instance* __restrict__ insts, const int32_t* __restrict__ work, const __grid_constant__ Lowered how) {
+  run_batched<true, 4>(P, insts, work, how);
 }
 
 // The same builds for launches of fewer CTAs than the GPU has SMs (single instances): each CTA's
@@ -2104,13 +2325,13 @@ __global__ void __launch_bounds__(PGX_MAX_THREADS_FFT) line_program_batched_fft(
 // loads a thread cost there more than they hide.
 __global__ void __launch_bounds__(PGX_MAX_THREADS) line_program_batched_lat(const __grid_constant__ pgx_program P,
                                                                             const pgx_instance* __restrict__ insts,
-                                                                            const int32_t* __restrict__ work, unsigned init) {
-  run_batched<false, 1>(P, insts, work, init);
+                                                                            const int32_t* __restrict__ work, const __grid_constant__ Lowered how) {
+  run_batched<false, 1>(P, insts, work, how);
 }
 
 __global__ void __launch_bounds__(PGX_MAX_THREADS_FFT) line_program_batched_fft_lat(
-    const __grid_constant__ pgx_program P, const pgx_instance* __restrict__ insts, const int32_t* __restrict__ work, unsigned init) {
-  run_batched<true, 1>(P, insts, work, init);
+    const __grid_constant__ pgx_program P, const pgx_instance* __restrict__ insts, const int32_t* __restrict__ work, const __grid_constant__ Lowered how) {
+  run_batched<true, 1>(P, insts, work, how);
 }
 
 }  // namespace pgx
@@ -2161,17 +2382,20 @@ static int raise_smem_cap(const void* fn, int which) {
   return e;
 }
 
-int launch_single(const pgx_program* P, const pgx_instance* I, cudaStream_t s, int ntiles) {
-  int64_t smem = pgx_program_smem(P);
-  const bool fft = pgx_has_dct(*P);
-  const unsigned init = pgx_init_mask(*P);
+int launch_single(const pgx_program* P0, const pgx_instance* I, cudaStream_t s, int ntiles) {
+  int64_t smem = pgx_program_smem(P0);
+  const bool fft = pgx_has_dct(*P0);
+  pgx_program low;
+  Lowered how;
+  pgx_lower(*P0, low, how);
+  const pgx_program* P = &low;
   if (smem > 48 * 1024) {
     int e = fft ? raise_smem_cap((const void*)line_program_single_fft, 2)
                 : raise_smem_cap((const void*)line_program_single, 0);
     if (e) return e;
   }
-  if (fft) line_program_single_fft<<<ntiles, P->nthreads, smem, s>>>(*P, *I, init);
-  else line_program_single<<<ntiles, P->nthreads, smem, s>>>(*P, *I, init);
+  if (fft) line_program_single_fft<<<ntiles, P->nthreads, smem, s>>>(*P, *I, how);
+  else line_program_single<<<ntiles, P->nthreads, smem, s>>>(*P, *I, how);
   return (int)cudaGetLastError();
 }
 
@@ -2225,11 +2449,14 @@ static int sm_count() {
   return count[dev];
 }
 
-int launch_batched(const pgx_program* P, const pgx_instance* d_insts, const int32_t* d_work, int nwork,
+int launch_batched(const pgx_program* P0, const pgx_instance* d_insts, const int32_t* d_work, int nwork,
                    cudaStream_t s) {
-  int64_t smem = pgx_program_smem(P) + ((sizeof(pgx_instance) + 15) / 16) * 16;
-  const bool fft = pgx_has_dct(*P);
-  const unsigned init = pgx_init_mask(*P);
+  int64_t smem = pgx_program_smem(P0) + ((sizeof(pgx_instance) + 15) / 16) * 16;
+  const bool fft = pgx_has_dct(*P0);
+  pgx_program low;
+  Lowered how;
+  pgx_lower(*P0, low, how);
+  const pgx_program* P = &low;
   const bool lat = nwork < sm_count();  // fewer CTAs than SMs: the latency build
   const void* fn = fft ? (lat ? (const void*)line_program_batched_fft_lat : (const void*)line_program_batched_fft)
                        : (lat ? (const void*)line_program_batched_lat : (const void*)line_program_batched);
@@ -2238,11 +2465,11 @@ int launch_batched(const pgx_program* P, const pgx_instance* d_insts, const int3
     if (e) return e;
   }
   if (fft) {
-    if (lat) line_program_batched_fft_lat<<<nwork, P->nthreads, smem, s>>>(*P, d_insts, d_work, init);
-    else line_program_batched_fft<<<nwork, P->nthreads, smem, s>>>(*P, d_insts, d_work, init);
+    if (lat) line_program_batched_fft_lat<<<nwork, P->nthreads, smem, s>>>(*P, d_insts, d_work, how);
+    else line_program_batched_fft<<<nwork, P->nthreads, smem, s>>>(*P, d_insts, d_work, how);
   } else {
-    if (lat) line_program_batched_lat<<<nwork, P->nthreads, smem, s>>>(*P, d_insts, d_work, init);
-    else line_program_batched<<<nwork, P->nthreads, smem, s>>>(*P, d_insts, d_work, init);
+    if (lat) line_program_batched_lat<<<nwork, P->nthreads, smem, s>>>(*P, d_insts, d_work, how);
+    else line_program_batched<<<nwork, P->nthreads, smem, s>>>(*P, d_insts, d_work, how);
   }
   return (int)cudaGetLastError();
 }
