@@ -117,6 +117,11 @@ enum pgx_dct_mode { PGX_DCT_RAW = 0, PGX_DCT_FWD = 1, PGX_DCT_BWD = 2, PGX_DCT_F
 /* op.k of DENSE: PGX_DENSE_MMA runs the contraction on the FP64 tensor cores (DMMA,
  * 8 x 8 x 4 tiles: rows x lines x columns) instead of one FMA chain per output. */
 #define PGX_DENSE_MMA 2
+/* op.k of DENSE: PGX_DENSE_TC contracts on the FP16 tensor cores in exact digits (fixed point: 63 bits of
+ * every row's and line's largest value, products summed to 2^-66 of the two).  The matrix at `mat` is
+ * followed by its digits: pgx_dense_pack writes them.  Programs with DCT ops, CTAs of more than 256
+ * threads and persistent launches run the FMA form of the same op. */
+#define PGX_DENSE_TC 4
 /* Largest CTA: 1024 threads, 768 for programs with DCT ops (their kernel is compiled for up
  * to 80 registers a thread; the kernel without the FFT code for 64). */
 #define PGX_MAX_THREADS 1024
@@ -347,6 +352,12 @@ int pgx_matrix_apply(const pgx_matrix_plan* plan, const double* in, int64_t in_s
                      void* stream);
 /* 1 if the plan is stored banded, 0 if dense. */
 int pgx_matrix_plan_is_banded(const pgx_matrix_plan* plan);
+
+/* A DENSE op's matrix for PGX_DENSE_TC, in DEVICE memory: `A` holds rows x cols doubles at the start of a
+ * 16-byte aligned buffer of pgx_dense_doubles(rows, cols) doubles, and pgx_dense_pack fills the rest with the
+ * matrix's digits (asynchronously on `stream`). */
+int64_t pgx_dense_doubles(int32_t rows, int32_t cols);
+int pgx_dense_pack(double* A, int32_t rows, int32_t cols, void* stream);
 
 /* Device table of DCT ops for line programs built by the host: twiddle factors of
  * the DCT-I of n points (2(n-1) complex values exp(-2 pi i k / (2(n-1))), then the

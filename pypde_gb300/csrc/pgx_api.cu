@@ -26,6 +26,7 @@ int persistent_shape(const pgx_program* progs, int nprogs, int threads, int* out
 int launch_persistent(const pgx_program* d_progs, int nprogs, const pgx_instance* d_descs, int ndescs,
                       const pgx_persist_item* d_items, int nitems, int32_t* d_counters, int ncounters,
                       int32_t* d_state, int ctas, int threads, int64_t smem, long long spin_limit, cudaStream_t s);
+int dense_pack(const double* d_A, int rows, int cols, void* d_packed, cudaStream_t s);
 }
 
 static thread_local int g_last_cuda = 0;
@@ -240,6 +241,19 @@ extern "C" int pgx_persist_error(const int32_t* d_state, int32_t* error, int32_t
 }
 
 // ------------------------------------------------------------ device tables
+// rows x cols doubles padded to an even count, 4 KB of digits for every 16 x 16 block, a scale per padded row
+extern "C" int64_t pgx_dense_doubles(int32_t rows, int32_t cols) {
+  if (rows < 1 || cols < 1) return 0;
+  const int64_t rt = (rows + 15) / 16, kt = (cols + 15) / 16;
+  return (((int64_t)rows * cols + 1) & ~(int64_t)1) + rt * kt * 512 + rt * 8;
+}
+
+extern "C" int pgx_dense_pack(double* A, int32_t rows, int32_t cols, void* stream) {
+  if (!A || ((uintptr_t)A & 15) || rows < 1 || cols < 1 || rows > PGX_LMAX || cols > PGX_LMAX) return PGX_E_ARG;
+  const int e = pgx::dense_pack(A, rows, cols, A + (((size_t)rows * cols + 1) & ~(size_t)1), (cudaStream_t)stream);
+  return e ? cuda_fail((cudaError_t)e) : PGX_OK;
+}
+
 namespace {
 std::mutex g_mu;
 
@@ -251,6 +265,22 @@ int upload(const std::vector<double>& h, double** d) {
   if (e != cudaSuccess) {
     cudaFree(p);
     return cuda_fail(e);
+  }
+  *d = (double*)p;
+  return PGX_OK;
+}
+
+// A dense matrix with the digits of PGX_DENSE_TC behind it.
+int upload_dense(const std::vector<double>& h, int rows, int cols, double** d) {
+  void* p = nullptr;
+  cudaError_t e = cudaMalloc(&p, (size_t)pgx_dense_doubles(rows, cols) * sizeof(double));
+  if (e != cudaSuccess) return cuda_fail(e);
+  e = cudaMemcpy(p, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice);
+  int rc = e == cudaSuccess ? pgx_dense_pack((double*)p, rows, cols, nullptr) : cuda_fail(e);
+  if (!rc && (e = cudaStreamSynchronize(nullptr)) != cudaSuccess) rc = cuda_fail(e);
+  if (rc) {
+    cudaFree(p);
+    return rc;
   }
   *d = (double*)p;
   return PGX_OK;
@@ -365,7 +395,7 @@ int dense_dct(int n, int mode, const double** out) {
       h[(size_t)k * n + j] = dct_post_h(mode, k, N) * c * dct_pre_h(mode, j, N);
     }
   double* d = nullptr;
-  int rc = upload(h, &d);
+  int rc = upload_dense(h, n, n, &d);
   if (rc) return rc;
   g_dense[key] = d;
   *out = d;
@@ -412,6 +442,19 @@ void pick_tile(pgx_program* P, int nlines, int maxlen, int nbuf, int fft_n) {
     int wt = 64 * tb;  // two chains (parities) per line, one warp each
     P->nthreads = wt < 256 ? 256 : (wt > PGX_MAX_THREADS ? PGX_MAX_THREADS : wt);
   }
+}
+
+// A LOAD, DENSE, STORE pass on the tensor cores, where that pays: an instruction takes eight lines whether they
+// are there or not, so a launch needs a few an SM to fill them (511 lines of 257 points 31 us against 72 us as
+// FP64 chains, 127 lines of 129 points 11 us against 8).  Eight lines a CTA (the launch splits the rows over
+// CTAs), a warp per row block up to eight.
+void dense_tile(pgx_program* P, int nlines, int rows) {
+  const int64_t most = (smem_optin_max() - 4096) / (16 * (int64_t)P->lcap);  // slot and spare
+  if (nlines < 3 * 152 || most < 8) return;
+  P->ops[1].k = (int16_t)(P->ops[1].k | PGX_DENSE_TC);
+  P->tb = 8;
+  const int rt = (rows + 15) / 16;
+  P->nthreads = 32 * (rt < 2 ? 2 : (rt > 8 ? 8 : rt));
 }
 
 pgx_op mk(int code, int a, int b = -1, int arr = -1, int mat = -1, int len = -1, int k = 0, double alpha = 1.0) {
@@ -472,6 +515,7 @@ int pgx_dct_pass(const double* in, int64_t in_s0, int64_t in_s1, int32_t n_in, d
   }
   P.ops[2] = mk(PGX_OP_STORE, 0, -1, 1);
   pick_tile(&P, nlines, n, 2, P.fft_n);
+  if (!fft && !mma) dense_tile(&P, nlines, n);
   if (mma) {  // one 8-line tensor-core tile per CTA, a warp per 8-row block
     P.tb = 8;
     P.nthreads = 32 * ((n + 7) / 8);
@@ -978,7 +1022,7 @@ extern "C" int pgx_matrix_plan_create(const double* A, int32_t rows, int32_t col
     p->ndiag = 0;
     tab.assign(A, A + (size_t)rows * cols);
   }
-  int rc = upload(tab, &p->tab);
+  int rc = p->banded ? upload(tab, &p->tab) : upload_dense(tab, rows, cols, &p->tab);
   if (rc) {
     delete p;
     return rc;
@@ -1018,5 +1062,6 @@ extern "C" int pgx_matrix_apply(const pgx_matrix_plan* p, const double* in, int6
   }
   P.ops[2] = mk(PGX_OP_STORE, 0, -1, 1);
   pick_tile(&P, nlines, p->rows > p->cols ? p->rows : p->cols, 2, 0);
+  if (!p->banded) dense_tile(&P, nlines, p->rows);
   return pgx_run(&P, &I, stream);
 }

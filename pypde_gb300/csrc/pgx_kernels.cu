@@ -118,6 +118,7 @@ struct Lowered {
   uint32_t merged;     // the program may hold merged ops
   int16_t fft_slots, fft_in_slot, fft_in_spare;  // pgx_fft_slots, pgx_fft_in_slot, pgx_fft_in_spare
   uint32_t mtb, mlcap;                           // multipliers of FastDiv for tb and lcap
+  int32_t parts;                                 // CTAs that share a tile's DENSE op (LOAD, DENSE, STORE programs)
 };
 }  // namespace pgx
 static_assert(PGX_MAX_OPS <= 96, "a barrier bit per op");
@@ -126,7 +127,7 @@ inline void pgx_lower(const pgx_program& P, pgx_program& out, pgx::Lowered& how)
   using namespace pgx;
   out = P;
   how = Lowered{pgx_init_mask(P), {0, 0, 0}, 1, (int16_t)pgx_fft_slots(P), pgx_fft_in_slot(P), pgx_fft_in_spare(P),
-                0xffffffffu / (uint32_t)P.tb + 1u, 0xffffffffu / (uint32_t)P.lcap + 1u};
+                0xffffffffu / (uint32_t)P.tb + 1u, 0xffffffffu / (uint32_t)P.lcap + 1u, 1};
   int n = 0;
   for (int o = 0; o < P.nops; ++o) {
     pgx_op op = P.ops[o];
@@ -454,7 +455,8 @@ __device__ void op_load_stencil(Ctx& c, const pgx_op& op, const pgx_instance& I,
 }
 
 template <int KU, bool ONE, bool ADD>
-__device__ __forceinline__ void store_loop(const Ctx& c, const View& v, const double* s, double alpha) {
+__device__ __forceinline__ void store_loop(const Ctx& c, const View& v, const double* s, double alpha, int i0 = 0,
+                                           int i1 = 1 << 30) {
   const int c_tb = c.tb;
   const int c_lcap = c.lcap;
   const int c_nthreads = c.nthreads;
@@ -479,7 +481,7 @@ __device__ __forceinline__ void store_loop(const Ctx& c, const View& v, const do
         if (contig) { t = fd.div(idx); i = idx - t * n; }
         else { i = fd.div(idx); t = idx - i * c_tb; }
         const int line = l0 + t;
-        if (line < nl) {
+        if (line < nl && i >= i0 && i < i1) {
           x[u] = s[t * c_lcap + i];
           dp[u] = v.p + (int64_t)i * v.se + (int64_t)line * v.sl;
           if (ADD) old[u] = *dp[u];
@@ -495,13 +497,19 @@ __device__ __forceinline__ void store_loop(const Ctx& c, const View& v, const do
   }
 }
 template <int KU>
-__device__ void op_store(const Ctx& c, const pgx_op& op, const pgx_instance& I, int axis, bool add) {
+__device__ void op_store(const Ctx& c, const pgx_op& op, const pgx_instance& I, int axis, bool add, int part = 0,
+                         int parts = 1) {
   const View v = view_of(I.arr[op.arr], axis);
   const double alpha = op_alpha(op, I);
   const double* s = slot_ptr(c, op.a);
   if (is_one(alpha)) {
     if (add) store_loop<KU, true, true>(c, v, s, alpha);
-    else store_loop<KU, true, false>(c, v, s, alpha);
+    else if (parts == 1) store_loop<KU, true, false>(c, v, s, alpha);
+    else {  // the row blocks of a split DENSE op
+      const int rt = (c.slen(op.a) + 15) >> 4;
+      store_loop<KU, true, false>(c, v, s, alpha, 16 * (rt * part / parts),
+                                  part + 1 == parts ? 1 << 30 : 16 * (rt * (part + 1) / parts));
+    }
   } else {
     if (add) store_loop<KU, false, true>(c, v, s, alpha);
     else store_loop<KU, false, false>(c, v, s, alpha);
@@ -1166,6 +1174,208 @@ __device__ void op_dense_mma(Ctx& c, const pgx_op& op, const pgx_instance& I) {
   c.set_slen(op.a, rows);
 }
 
+// ------------------------------------------------ dense operators on the FP16 tensor cores
+// y = A x in fixed point, exactly up to the digits kept: the rows of A and the lines of x are integers of 63
+// bits on a scale of their own (the row's, the line's largest value), written in eight balanced base-256
+// digits, which FP16 holds exactly.  Products of two digits are below 2^14, so the tensor cores' FP32 sums
+// of 8 such products over 128 columns stay whole numbers up to 2^24; the sums of each weight 256^(i+j)
+// (i + j >= 6: 43 of the 64 digit pairs; the rest is below 2^-66 of the two scales a column) then go to 32-bit
+// integers, and the weights' sums to one 64-bit number and a double.
+//
+// Against FP64: a row of 255 columns on two lines took 137,000 cycles of a CTA at the FP64 pipe's ~66 cycles
+// a warp instruction; here a 16 x 16 block of A times 8 lines is 43 m16n8k16 instructions and 4 KB of digits
+// from L2.  mma.sync and not tcgen05: the operands are a handful of lines a CTA, whose digits are cut from
+// the slot in registers, and the tensor pipe is not what bounds it at that shape.
+//
+// Packed operand (pgx_dense_pack), after the rows x cols doubles (padded to an even count): for every 16 x 16
+// block, row block by row block, 8 digits (the least first) of 32 lanes' A fragments of m16n8k16, 16 bytes
+// each; then an int32 scale per padded row (kDenseBad: a NaN or an infinity in it).
+// High word of |x_j| of a line read as integers
+__device__ __forceinline__ uint32_t fx_hi(const int64_t* x, int j) {
+  return (uint32_t)((uint64_t)x[j] >> 32) & 0x7fffffffu;
+}
+constexpr int kDenseBad = 1 << 20;
+__device__ __forceinline__ void hmma_16x8x16(float (&d)[4], const uint4& a, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+               "{%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
+}
+constexpr uint64_t kDigitBias = 0x8080808080808080ULL;  // balanced digits are the biased number's bytes less 128
+// digit i of two biased numbers as a pair of FP16: 1024 + byte is 0x6400 | byte, less 1152
+template <int i>
+__device__ __forceinline__ uint32_t digit_pair(uint64_t a, uint64_t b) {
+  const uint32_t wa = i < 4 ? (uint32_t)a : (uint32_t)(a >> 32), wb = i < 4 ? (uint32_t)b : (uint32_t)(b >> 32);
+  const uint32_t p = __byte_perm(wa, wb, (i & 3) | ((4 + (i & 3)) << 8)) & 0x00ff00ffu;
+  uint32_t r;
+  asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(p | 0x64006400u), "r"(0x64806480u));
+  return r;
+}
+__device__ __forceinline__ uint32_t digit_pair(int i, uint64_t a, uint64_t b) {
+  switch (i) {
+    case 0: return digit_pair<0>(a, b);
+    case 1: return digit_pair<1>(a, b);
+    case 2: return digit_pair<2>(a, b);
+    case 3: return digit_pair<3>(a, b);
+    case 4: return digit_pair<4>(a, b);
+    case 5: return digit_pair<5>(a, b);
+    case 6: return digit_pair<6>(a, b);
+    default: return digit_pair<7>(a, b);
+  }
+}
+// Scale E of numbers whose largest high word (without sign) is hm: all of them below 2^E; kDenseBad
+__device__ __forceinline__ int dense_scale(uint32_t hm) {
+  return hm >= 0x7ff00000u ? kDenseBad : max((int)(hm >> 20), 1) - 1022;
+}
+// x 2^(62 - E), rounded
+__device__ __forceinline__ int64_t dense_int(double x, int E) { return fx_from_double(x, FX_P0 - 62 + E, 0, 0); }
+
+__global__ void dense_pack_scales(const double* __restrict__ A, int rows, int cols, int32_t* __restrict__ scale, int padded) {
+  const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= padded) return;
+  uint32_t hm = 0;
+  if (r < rows)
+    for (int k = lane; k < cols; k += 32) hm = max(hm, fx_hi(reinterpret_cast<const int64_t*>(A) + (size_t)r * cols, k));
+  for (int o = 16; o > 0; o >>= 1) hm = max(hm, __shfl_xor_sync(FULLMASK, hm, o));
+  if (lane == 0) scale[r] = dense_scale(hm);
+}
+__global__ void dense_pack_digits(const double* __restrict__ A, int rows, int cols, const int32_t* __restrict__ scale,
+                                  uint4* __restrict__ out, int kt) {
+  const int block = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int rt = (rows + 15) >> 4;
+  if (block >= rt * kt) return;
+  const int r0 = (block / kt) * 16 + (lane >> 2), k0 = (block % kt) * 16 + 2 * (lane & 3);
+  uint64_t v[2][4];  // rows r0, r0 + 8; columns k0, k0 + 1, k0 + 8, k0 + 9
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int r = r0 + 8 * h, k = k0 + (q & 1) + 8 * (q >> 1);
+      int64_t x = 0;
+      if (r < rows && k < cols && scale[r] != kDenseBad) x = dense_int(A[(size_t)r * cols + k], scale[r]);
+      v[h][q] = (uint64_t)x + kDigitBias;
+    }
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    out[((size_t)block * 8 + i) * 32 + lane] = make_uint4(digit_pair(i, v[0][0], v[0][1]), digit_pair(i, v[1][0], v[1][1]),
+                                                          digit_pair(i, v[0][2], v[0][3]), digit_pair(i, v[1][2], v[1][3]));
+}
+
+// Part `part` of `parts` of the row blocks (the other parts of a tile are other CTAs').
+__device__ void op_dense_tc(Ctx& c, const pgx_op& op, const pgx_instance& I, int part, int parts) {
+  const int tb = c.tb, lcap = c.lcap;
+  const double* A = I.mat[op.mat];
+  const int rows = I.len[op.len], cols = c.slen(op.a);
+  const int rt = (rows + 15) >> 4, kt = (cols + 15) >> 4;
+  const uint4* digits = reinterpret_cast<const uint4*>(A + (((size_t)rows * cols + 1) & ~(size_t)1));
+  const int32_t* rscale = reinterpret_cast<const int32_t*>(digits + (size_t)rt * kt * 256);
+  int64_t* x = reinterpret_cast<int64_t*>(slot_ptr(c, op.a));
+  int64_t* y = reinterpret_cast<int64_t*>(spare_ptr(c));
+  const int lane = c.tid & 31, warp = c.tid >> 5, nw = c.nthreads >> 5;
+  const int nlb = (tb + 7) >> 3;
+  const int r0 = rt * part / parts, nrt = rt * (part + 1) / parts - r0;
+  // A block's 4 KB are one prefetch a lane: the warp asks for its first ones while the lines become integers,
+  // then for every block two ahead (loading ahead into registers instead took 184 of them, and one CTA an SM
+  // where two fit: 513 x 257, H_y 47 us against 31).
+  if (warp < nrt * nlb)
+    for (int kb = 0; kb < 2 && kb < kt; ++kb)
+      prefetch_l1(reinterpret_cast<const double*>(digits + ((size_t)(r0 + warp % nrt) * kt + kb) * 256 + 8 * lane));
+  // the lines as integers, in place; a line's scale waits in the last point of its result, which no row has
+  const LineLanes g = line_lanes(c, tb);
+  for (int base = g.first; base < tb; base += g.stride) {
+    const int t = base + g.grp;
+    const bool valid = t < tb;
+    int64_t* xl = x + (valid ? t : 0) * lcap;
+    uint32_t hm = 0;
+    if (valid)
+      for (int k = g.sub; k < cols; k += g.L) hm = max(hm, fx_hi(xl, k));
+    for (int o = g.L >> 1; o > 0; o >>= 1) hm = max(hm, __shfl_xor_sync(FULLMASK, hm, o, g.L));
+    if (!valid) continue;
+    const int E = dense_scale(hm);
+    if (E != kDenseBad)
+      for (int k = g.sub; k < cols; k += g.L) xl[k] = dense_int(fx_double((uint64_t)xl[k]), E);
+    if (g.sub == 0) y[t * lcap + lcap - 1] = E;
+  }
+  __syncthreads();
+  const int gr = lane >> 2, q = lane & 3;
+  for (int blk = warp; blk < nrt * nlb; blk += nw) {  // warp-uniform loop
+    const int lb = blk / nrt, rb = r0 + blk - lb * nrt;
+    const int t = lb * 8 + gr;  // the line whose digits this lane cuts
+    const int64_t* xl = x + (t < tb ? t : 0) * lcap;
+    const bool tok = t < tb && (int)y[(t < tb ? t : 0) * lcap + lcap - 1] != kDenseBad;
+    const uint4* ap = digits + (size_t)rb * kt * 256 + lane;
+    float f[9][4];
+    int64_t hi[4], lo[4];  // sums of the weights 4 to 8 and 0 to 3
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      hi[e] = lo[e] = 0;
+#pragma unroll
+      for (int w = 0; w < 9; ++w) f[w][e] = 0.0f;
+    }
+    for (int kb = 0; kb < kt; ++kb, ap += 256) {
+      uint4 a[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) a[i] = __ldg(ap + 32 * i);
+      if (kb + 2 < kt) prefetch_l1(reinterpret_cast<const double*>(ap + 512 - lane + 8 * lane));
+      const int k = kb * 16 + 2 * q;
+      uint64_t v[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int kk = k + (e & 1) + 8 * (e >> 1);
+        v[e] = (uint64_t)(tok && kk < cols ? xl[kk] : 0) + kDigitBias;
+      }
+#pragma unroll
+      for (int j = 7; j >= 0; --j) {  // the many sums first: neighbouring instructions have different ones
+        const uint32_t b0 = digit_pair(j, v[0], v[1]), b1 = digit_pair(j, v[2], v[3]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if (i + j >= 6) hmma_16x8x16(f[i + j >= 6 ? i + j - 6 : 0], a[i], b0, b1);
+      }
+      if ((kb & 7) == 7 || kb == kt - 1) {  // 128 columns: the sums are still whole
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          int64_t h = 0, l = 0;
+#pragma unroll
+          for (int w = 8; w >= 4; --w) h = (h << 8) + __float2int_rn(f[w][e]);
+#pragma unroll
+          for (int w = 3; w >= 0; --w) l = (l << 8) + __float2int_rn(f[w][e]);
+          hi[e] += h;
+          lo[e] += l;
+#pragma unroll
+          for (int w = 0; w < 9; ++w) f[w][e] = 0.0f;
+        }
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int r = rb * 16 + gr + 8 * (e >> 1), to = lb * 8 + 2 * q + (e & 1);
+      if (r >= rows || to >= tb) continue;
+      // hi 2^32 + lo as its 63 leading bits and a power of two; lo is below 2^53: it adds at most 2^21 to hi
+      const int room = fx_clz((uint64_t)(hi[e] < 0 ? ~hi[e] : hi[e])) - 2;
+      const int up = max(0, min(room, 32));
+      const int64_t sum = (int64_t)((uint64_t)hi[e] << up) + (lo[e] >> (32 - up));
+      const int Er = rscale[r], El = (int)y[to * lcap + lcap - 1];
+      double res;
+      if (Er != kDenseBad && El != kDenseBad) {
+        // digits stand for 2^(E - 62), the lowest weight for 256^6
+        res = fx_to_double(sum, Er + El - 124 + 48 + 32 - up);
+      } else {  // a NaN or an infinity: the plain sum of products
+        const double* Ar = A + (size_t)r * cols;
+        res = 0.0;
+        for (int k = 0; k < cols; ++k) {
+          const int64_t xi = x[to * lcap + k];
+          res = fma(Ar[k], El == kDenseBad ? fx_double((uint64_t)xi) : fx_to_double(xi, El - 62), res);
+        }
+      }
+      y[to * lcap + r] = (int64_t)fx_bits(res);
+    }
+  }
+  __syncthreads();
+  zero_tail(c, spare_ptr(c), rows);
+  swap_spare(c, op.a);
+  c.set_slen(op.a, rows);
+}
+
 __device__ void op_dense(Ctx& c, const pgx_op& op, const pgx_instance& I) {
   const int c_tb = c.tb;
   const int c_lcap = c.lcap;
@@ -1699,9 +1909,6 @@ __device__ __forceinline__ int fx_fft_any(const FxSlots& m, const FxSet& g, FxBu
 // Sum of absolute values of a line (n points), this lane's share, in FP32 over the high words (the low
 // ones add less than 2^-20 of it): the double's exponent field moves into the float's, `shift` further
 // down, clamped at zero and near the top.
-__device__ __forceinline__ uint32_t fx_hi(const int64_t* x, int j) {
-  return (uint32_t)((uint64_t)x[j] >> 32) & 0x7fffffffu;
-}
 __device__ __forceinline__ float fx_abs_part(uint32_t hi, int shift) {
   return __int_as_float(__viaddmin_s32_relu((int)hi, -shift, 254 << 20) << 3);
 }
@@ -2119,8 +2326,9 @@ __device__ void dct_paired_slot(Ctx& c, int slot, const pgx_op& op, const pgx_in
 
 // ------------------------------------------------------------------ driver
 // One tile of one instance: the program's ops on shared-memory slots that start at `sm`.
-template <bool FFT, int KU>
-__device__ void run_program(const pgx_program& P, const pgx_instance& I, int tile, int sm, const Lowered& how) {
+template <bool FFT, int KU, bool TC = false>
+__device__ void run_program(const pgx_program& P, const pgx_instance& I, int tile, int sm, const Lowered& how,
+                            int part = 0) {
   Ctx c;
   c.tb = P.tb;
   c.lcap = P.lcap;
@@ -2157,7 +2365,7 @@ __device__ void run_program(const pgx_program& P, const pgx_instance& I, int til
       case PGX_OP_LOAD: op_load<KU>(c, op, I, P.axis, 0); break;
       case PGX_OP_LOAD_ADD: op_load<KU>(c, op, I, P.axis, 1); break;
       case PGX_OP_LOAD_MUL: op_load<KU>(c, op, I, P.axis, 2); break;
-      case PGX_OP_STORE: op_store<KU>(c, op, I, P.axis, false); break;
+      case PGX_OP_STORE: op_store<KU>(c, op, I, P.axis, false, TC ? part : 0, TC ? how.parts : 1); break;
       case PGX_OP_STORE_ADD: op_store<KU>(c, op, I, P.axis, true); break;
       case PGX_OP_SCALE:
       case PGX_OP_AXPY:
@@ -2189,7 +2397,10 @@ __device__ void run_program(const pgx_program& P, const pgx_instance& I, int til
         }
         break;
       case PGX_OP_BANDED: op_banded<KU>(c, op, I); break;
-      case PGX_OP_DENSE: op_dense(c, op, I); break;
+      case PGX_OP_DENSE:
+        if (TC && (op.k & PGX_DENSE_TC)) op_dense_tc(c, op, I, part, how.parts);
+        else op_dense(c, op, I);
+        break;
       case PGX_OP_FDMA: op_fdma(c, op, I, false); break;
       case PGX_OP_POISSON: op_fdma(c, op, I, true); break;
       case PGX_OP_DIFF_T: op_diff_t(c, op); break;
@@ -2204,17 +2415,19 @@ __device__ void run_program(const pgx_program& P, const pgx_instance& I, int til
   }
 }
 
-template <bool FFT, int KU>
+template <bool FFT, int KU, bool TC = false>
 __device__ __forceinline__ void run_batched(const pgx_program& P, const pgx_instance* __restrict__ insts,
                                             const int32_t* __restrict__ work, const Lowered& how) {
   pgx_instance* sI = reinterpret_cast<pgx_instance*>(smem_dyn);
-  const int inst = work[2 * blockIdx.x], tile = work[2 * blockIdx.x + 1];
+  const int item = TC ? blockIdx.x / how.parts : blockIdx.x;
+  const int inst = work[2 * item], tile = work[2 * item + 1];
   const int nwords = sizeof(pgx_instance) / 8;
   const double* src = reinterpret_cast<const double*>(insts + inst);
   double* dst = reinterpret_cast<double*>(sI);
   for (int i = threadIdx.x; i < nwords; i += blockDim.x) dst[i] = src[i];
   __syncthreads();
-  run_program<FFT, KU>(P, *sI, tile, (int)((sizeof(pgx_instance) + 15) / 16 * 2), how);
+  run_program<FFT, KU, TC>(P, *sI, tile, (int)((sizeof(pgx_instance) + 15) / 16 * 2), how,
+                       TC ? blockIdx.x - item * how.parts : 0);
 }
 
 // ------------------------------------------------------------- persistent steps
@@ -2288,7 +2501,7 @@ __global__ void __launch_bounds__(PGX_MAX_THREADS_FFT) line_program_persistent(
     __syncthreads();
     run_program<true, 4>(*sP, *sI, w.tile, kPersistHead / 8,
                          Lowered{~0u, {0, 0, 0}, 0, (int16_t)pgx_fft_slots(*sP), pgx_fft_in_slot(*sP),
-                                 pgx_fft_in_spare(*sP), c_divs.m[sP->tb], c_divs.m[sP->lcap]});
+                                 pgx_fft_in_spare(*sP), c_divs.m[sP->tb], c_divs.m[sP->lcap], 1});
     // run_program ends every op with a block barrier: every store of the tile is done here
     if (threadIdx.x == 0) {
       __threadfence();
@@ -2334,6 +2547,21 @@ __global__ void __launch_bounds__(PGX_MAX_THREADS_FFT) line_program_batched_fft_
   run_batched<true, 1>(P, insts, work, how);
 }
 
+// The builds with the tensor-core DENSE op, for programs that have one and no DCT: its 36 sums, 32 registers of
+// digits and eight 64-bit totals take more registers than the others' CTA sizes leave; two such CTAs fit an SM.
+constexpr int kMaxThreadsTc = 256;
+__global__ void __launch_bounds__(kMaxThreadsTc, 2) line_program_single_tc(const __grid_constant__ pgx_program P,
+                                                                        const __grid_constant__ pgx_instance I,
+                                                                        const __grid_constant__ Lowered how) {
+  run_program<false, 1, true>(P, I, blockIdx.x / how.parts, 0, how, blockIdx.x % how.parts);
+}
+__global__ void __launch_bounds__(kMaxThreadsTc, 2) line_program_batched_tc(const __grid_constant__ pgx_program P,
+                                                                         const pgx_instance* __restrict__ insts,
+                                                                         const int32_t* __restrict__ work,
+                                                                         const __grid_constant__ Lowered how) {
+  run_batched<false, 1, true>(P, insts, work, how);
+}
+
 }  // namespace pgx
 
 // ---------------------------------------------------------------------------
@@ -2357,7 +2585,7 @@ namespace pgx {
 // could invalidate by setting a lower value.
 static int raise_smem_cap_once(const void* fn, int which) {
   static std::mutex mu;
-  static bool done[7][64] = {};
+  static bool done[9][64] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return (int)e;
@@ -2382,6 +2610,40 @@ static int raise_smem_cap(const void* fn, int which) {
   return e;
 }
 
+// SMs of the current device, looked up once per device.
+static int sm_count() {
+  static std::mutex mu;
+  static int count[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  std::lock_guard<std::mutex> lk(mu);
+  if (count[dev] == 0 && cudaDeviceGetAttribute(&count[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    cudaGetLastError();
+    count[dev] = 0;
+  }
+  return count[dev];
+}
+
+// Whether a lowered program runs in the build with the tensor-core DENSE op.
+static bool pgx_use_tc(const pgx_program& P) {
+  if (P.nthreads > kMaxThreadsTc || pgx_has_dct(P)) return false;
+  for (int o = 0; o < P.nops; ++o)
+    if (P.ops[o].code == PGX_OP_DENSE && (P.ops[o].k & PGX_DENSE_TC)) return true;
+  return false;
+}
+// CTAs per tile of a LOAD, DENSE, STORE program: a DENSE op's row blocks are independent, and a launch of
+// fewer tiles than SMs leaves the others idle (511 x 511 on 64 tiles of 8 lines).  The loads and the cut into
+// digits are repeated in every part, so two CTAs an SM are the most, and two row blocks a part the least.
+static int pgx_dense_parts(const pgx_program& P, int tiles, int sms) {
+  if (P.nops != 3 || P.ops[0].code != PGX_OP_LOAD || P.ops[1].code != PGX_OP_DENSE || P.ops[2].code != PGX_OP_STORE ||
+      P.ops[0].a != P.ops[1].a || P.ops[1].a != P.ops[2].a || P.ops[2].par >= 0 || P.ops[2].alpha != 1.0 || tiles < 1)
+    return 1;
+  const int rt = (P.lcap + 15) / 16, most = rt / 2;
+  int parts = 2 * sms / tiles;
+  if (parts > most) parts = most;
+  return parts < 1 ? 1 : parts;
+}
+
 int launch_single(const pgx_program* P0, const pgx_instance* I, cudaStream_t s, int ntiles) {
   int64_t smem = pgx_program_smem(P0);
   const bool fft = pgx_has_dct(*P0);
@@ -2389,12 +2651,16 @@ int launch_single(const pgx_program* P0, const pgx_instance* I, cudaStream_t s, 
   Lowered how;
   pgx_lower(*P0, low, how);
   const pgx_program* P = &low;
+  const bool tc = pgx_use_tc(low);
+  if (tc) how.parts = pgx_dense_parts(low, ntiles, sm_count());
+  const void* fn = fft ? (const void*)line_program_single_fft
+                       : (tc ? (const void*)line_program_single_tc : (const void*)line_program_single);
   if (smem > 48 * 1024) {
-    int e = fft ? raise_smem_cap((const void*)line_program_single_fft, 2)
-                : raise_smem_cap((const void*)line_program_single, 0);
+    const int e = raise_smem_cap(fn, fft ? 2 : (tc ? 7 : 0));
     if (e) return e;
   }
   if (fft) line_program_single_fft<<<ntiles, P->nthreads, smem, s>>>(*P, *I, how);
+  else if (tc) line_program_single_tc<<<ntiles * how.parts, P->nthreads, smem, s>>>(*P, *I, how);
   else line_program_single<<<ntiles, P->nthreads, smem, s>>>(*P, *I, how);
   return (int)cudaGetLastError();
 }
@@ -2435,20 +2701,6 @@ int launch_persistent(const pgx_program* d_progs, int nprogs, const pgx_instance
   return (int)cudaGetLastError();
 }
 
-// SMs of the current device, looked up once per device.
-static int sm_count() {
-  static std::mutex mu;
-  static int count[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  std::lock_guard<std::mutex> lk(mu);
-  if (count[dev] == 0 && cudaDeviceGetAttribute(&count[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
-    cudaGetLastError();
-    count[dev] = 0;
-  }
-  return count[dev];
-}
-
 int launch_batched(const pgx_program* P0, const pgx_instance* d_insts, const int32_t* d_work, int nwork,
                    cudaStream_t s) {
   int64_t smem = pgx_program_smem(P0) + ((sizeof(pgx_instance) + 15) / 16) * 16;
@@ -2457,20 +2709,34 @@ int launch_batched(const pgx_program* P0, const pgx_instance* d_insts, const int
   Lowered how;
   pgx_lower(*P0, low, how);
   const pgx_program* P = &low;
+  const bool tc = pgx_use_tc(low);
+  if (tc) how.parts = pgx_dense_parts(low, nwork, sm_count());
   const bool lat = nwork < sm_count();  // fewer CTAs than SMs: the latency build
   const void* fn = fft ? (lat ? (const void*)line_program_batched_fft_lat : (const void*)line_program_batched_fft)
                        : (lat ? (const void*)line_program_batched_lat : (const void*)line_program_batched);
+  if (tc) fn = (const void*)line_program_batched_tc;
   if (smem > 48 * 1024) {
-    int e = raise_smem_cap(fn, fft ? (lat ? 6 : 3) : (lat ? 5 : 1));
+    int e = raise_smem_cap(fn, tc ? 8 : (fft ? (lat ? 6 : 3) : (lat ? 5 : 1)));
     if (e) return e;
   }
-  if (fft) {
+  if (tc) {
+    line_program_batched_tc<<<nwork * how.parts, P->nthreads, smem, s>>>(*P, d_insts, d_work, how);
+  } else if (fft) {
     if (lat) line_program_batched_fft_lat<<<nwork, P->nthreads, smem, s>>>(*P, d_insts, d_work, how);
     else line_program_batched_fft<<<nwork, P->nthreads, smem, s>>>(*P, d_insts, d_work, how);
   } else {
     if (lat) line_program_batched_lat<<<nwork, P->nthreads, smem, s>>>(*P, d_insts, d_work, how);
     else line_program_batched<<<nwork, P->nthreads, smem, s>>>(*P, d_insts, d_work, how);
   }
+  return (int)cudaGetLastError();
+}
+
+int dense_pack(const double* d_A, int rows, int cols, void* d_packed, cudaStream_t s) {
+  const int rt = (rows + 15) / 16, kt = (cols + 15) / 16;
+  uint4* digits = (uint4*)d_packed;
+  int32_t* scale = (int32_t*)(digits + (size_t)rt * kt * 256);
+  dense_pack_scales<<<rt * 2, 256, 0, s>>>(d_A, rows, cols, scale, rt * 16);
+  dense_pack_digits<<<(rt * kt + 7) / 8, 256, 0, s>>>(d_A, rows, cols, scale, digits, kt);
   return (int)cudaGetLastError();
 }
 }  // namespace pgx

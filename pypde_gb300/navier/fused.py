@@ -611,6 +611,24 @@ def dense_dct_host(n):
             "dct_fwd_t": np.ascontiguousarray(fwd.T)}
 
 
+def dense_dev(A):
+    """A dense operator on the device with its digits for the tensor cores behind it (pgx_dense_pack)."""
+    rows, cols = A.shape
+    L = _lib.lib()
+    buf = torch.empty(L.pgx_dense_doubles(rows, cols), dtype=DTYPE, device=device())
+    buf[:rows * cols].copy_(torch.from_numpy(np.ascontiguousarray(A)).reshape(-1))
+    _lib.check(L.pgx_dense_pack(buf.data_ptr(), rows, cols, stream()), "dense pack")
+    return buf
+
+
+DENSE_TABLES = ("Hy", "Qy", "HyT", "QyT")
+
+
+def tables_dev(host):
+    """Host operator tables on the device (the dense ones with their digits)."""
+    return {k: dense_dev(v) if k in DENSE_TABLES else to_dev(v) for k, v in host.items()}
+
+
 _DENSE_DCT_CACHE = {}
 
 
@@ -618,7 +636,7 @@ def _dense_dct_tables(n):
     """Dense DCT matrices of length n on the current device, shared by every instance."""
     key = (torch.cuda.current_device(), n)
     if key not in _DENSE_DCT_CACHE:
-        _DENSE_DCT_CACHE[key] = {k: to_dev(v) for k, v in dense_dct_host(n).items()}
+        _DENSE_DCT_CACHE[key] = {k: dense_dev(v) for k, v in dense_dct_host(n).items()}
     return _DENSE_DCT_CACHE[key]
 
 
@@ -752,7 +770,7 @@ class _Instance:
         g = _global_tables()
         t = {"sten_CD": g["sten_CD"], "sten_CN": g["sten_CN"], "tdma_CD": g["tdma_CD"]}
         host = host_tables(N, M, ns.T.xs[0].id, ns.dt * bt, ns.nu, ns.kappa, ns.scale, ns.solver_P._fd)
-        t.update({k: to_dev(v) for k, v in host.items()})
+        t.update(tables_dev(host))
         self.tables = t
         # per stage: parameters, ADI tables (lambda = dt a nu or dt a kappa) and the velocity arrays
         # of the stage and of the previous one (RK3)
@@ -910,6 +928,13 @@ def _pick(prog, lines_total, lcap, fft_n, max_lines):
     if fft_n > 1:
         tb = min(max(tb, 2), max(2, tbmax - tbmax % 2))
         tb -= tb % 2
+    elif _dense_tc(prog, lines_total, 256, fft_n, False):
+        # eight lines an instruction, there or not: eight a CTA where the launch splits the rows over CTAs
+        # (LOAD, DENSE, STORE), else as many as still leave every SM a CTA
+        tb = 8 if len(prog.ops) == 3 else 1
+        while tb < 8 and -(-lines_total // tb) > 152:
+            tb *= 2
+        tb = min(tb, tbmax)
     # one thread per (slot, line, parity) chain of the widest chain op
     width = 1
     for o in prog.ops:
@@ -924,6 +949,18 @@ def _pick(prog, lines_total, lcap, fft_n, max_lines):
     if wc:
         nt = max(256, min(ntmax, 32 * width * tb))
     return tb, min(nt, ntmax), bool(wc), sd, False
+
+
+# Dense operators go to the tensor cores in digits (PGX_DENSE_TC) in launches of at least this many lines and CTAs
+# of at most that many threads.  An instruction takes eight lines, so a launch needs a few lines an SM to fill
+# them: 511 lines of 257 points 31 us against 72 as FP64 chains, 127 lines of 129 points 11 against 8.
+DENSE_TC_LINES = 3 * 152
+MAX_THREADS_DENSE = 256
+
+
+def _dense_tc(prog, lines_total, nt, fft_n, dm):
+    return (lines_total >= DENSE_TC_LINES and nt <= MAX_THREADS_DENSE and (fft_n <= 1 or dm or not prog.has_dct)
+            and (dm or any(o.code == _lib.OP["DENSE"] for o in prog.ops)))
 
 
 def _max_threads(prog, fft_n, dm):
@@ -1006,9 +1043,10 @@ def launch_ops(prog, sd=False, dm=False):
     return ops
 
 
-def launch_program(prog, key, tb, nt, wc=False, sd=False, dm=False):
+def launch_program(prog, key, tb, nt, wc=False, sd=False, dm=False, tc=False):
     """The PgxProgram of one launch of ``prog`` for the size class ``key`` = (lcap, fft_n) with
-    ``tb`` lines and ``nt`` threads a CTA (``wc``, ``sd``, ``dm`` as in ``FusedBatch._group_launch``).
+    ``tb`` lines and ``nt`` threads a CTA (``wc``, ``sd``, ``dm`` as in ``FusedBatch._group_launch``;
+    ``tc``: its DENSE ops in digits on the FP16 tensor cores, PGX_DENSE_TC).
     One-slot transforms of the pass's (dealiased) length on even tiles run in the slots' own lines
     (PGX_DCT_SLOT): no FFT buffers of shared memory."""
     lcap, fft_n = key
@@ -1027,6 +1065,8 @@ def launch_program(prog, key, tb, nt, wc=False, sd=False, dm=False):
             P.ops[i].k = o.k | _lib.CHAIN_WARP
         if in_slot and o.code == _lib.OP["DCT"]:
             P.ops[i].k = o.k | _lib.DCT_SLOT
+        if tc and o.code == _lib.OP["DENSE"]:  # every dense table carries its digits (dense_dev)
+            P.ops[i].k = (o.k & ~_lib.DENSE_MMA) | _lib.DENSE_TC
     return P
 
 
@@ -1121,8 +1161,9 @@ class FusedBatch:
         """One launch of ``prog`` over ``members``; ``wc``: chain ops in warp-per-chain mode;
         ``sd``: multi-slot DCT ops as one op per slot; ``dm``: DCT ops as dense matrices and every
         DENSE op on the FP64 tensor cores (no FFT buffers)."""
-        P = launch_program(prog, key, tb, nt, wc, sd, dm)
         nv = len(prog.variants)
+        lines_total = sum(self.insts[k].lines(prog) for k in members) * nv
+        P = launch_program(prog, key, tb, nt, wc, sd, dm, _dense_tc(prog, lines_total, nt, key[1], dm))
         # the batched launch cannot read its descriptors on the host: check every member's host copy
         host = getattr(d_insts, "pgx_host", None)
         if host is None:

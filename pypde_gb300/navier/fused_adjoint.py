@@ -44,7 +44,7 @@ import torch
 from .. import _lib
 from .._dev import DTYPE, device, to_dev
 from .fused import (L_M, L_MD, L_MG, L_N, L_ND, L_NG, P_B, P_C, P_DT, P_EDT, P_EDU, P_IDT, P_ISX, P_ISZ, P_MDT,
-                    P_MDTSX, P_MDTSZ, P_MNU, P_TF, FusedBatch, Prog, _Instance, build_programs, host_tables)
+                    P_MDTSX, P_MDTSZ, P_MNU, P_TF, FusedBatch, Prog, _Instance, build_programs, host_tables, tables_dev)
 
 BAR_STATE = ("bUG", "bVG", "bTG", "bPG", "bPRES")
 
@@ -393,8 +393,7 @@ def add_adjoint_buffers(I, bar_views, beta=False):
             st.update(carry)
     host = host_tables(N, M, ns.T.xs[0].id, ns.dt * float(ns.beta), ns.nu, ns.kappa, ns.scale, ns.solver_P._fd,
                        adjoint=True)
-    for k in ("BxT", "ByT", "BSx_UT", "BSx_TT", "BSyT", "HyT", "QyT"):
-        I.tables[k] = to_dev(host[k])
+    I.tables.update(tables_dev({k: host[k] for k in ("BxT", "ByT", "BSx_UT", "BSx_TT", "BSyT", "HyT", "QyT")}))
 
 
 class FusedAdjoint(FusedBatch):
