@@ -404,17 +404,82 @@ int dense_dct(int n, int mode, const double** out) {
 
 int round_odd(int x) { return x | 1; }
 
+// Whether the folded transform of n points runs in its slot's own lines and the spare (PGX_DCT_SLOT): n - 1 =
+// 2^a 3^b with a >= 2, or a = 1 and b even (an odd number of stages is then to be had).
+bool dct_in_slot_ok(int n) {
+  int a = 0, b = 0, m = n - 1;
+  for (; m > 0 && m % 2 == 0; m /= 2) ++a;
+  for (; m > 0 && m % 3 == 0; m /= 3) ++b;
+  return m == 1 && (a >= 2 || (a == 1 && b % 2 == 0));
+}
+
+// Tile of a pass with an FFT.  A CTA's stages are separated by barriers, so an SM is filled by CTAs that wait at
+// different ones, not by wide CTAs: the smallest tile whose CTAs are all resident at once with three warps or more
+// each (the FFT build holds PGX_MAX_THREADS_FFT threads an SM, shared memory so many CTAs), at most a thread a
+// point and 384.  1025 lines of 1025 points in pairs of 192 threads 32 us (256 threads, a second wave: 37; six
+// lines and 512 threads, 171 CTAs on 152 SMs: 61), 769 x 769 21.7 against 24.2, up to 385 lines the same; 5000
+// lines of 65 points in sixes of 128 threads 12.7 (pairs: 19).  Launches that fill the GPU several times over run
+// 16 points a thread, where threads and shared memory run out together: 20000 lines of 129 points in tiles of 16
+// 48 us (pairs: 85), of 1025 in tiles of 4 482 (pairs: 517).  The transform in the
+// slot needs half the memory: 1537 x 1000 in pairs 53 us against 72.
+void pick_fft_tile(pgx_program* P, int nlines, bool warp_chains) {
+  if (dct_in_slot_ok(P->fft_n))
+    for (int o = 0; o < P->nops; ++o)
+      if (P->ops[o].code == PGX_OP_DCT) P->ops[o].k = (int16_t)(P->ops[o].k | PGX_DCT_SLOT);
+  const int N = P->fft_n - 1;
+  for (P->tb = 2; P->tb <= 16; P->tb += 2) {
+    const int64_t room = (smem_optin_max() + 1024) / (pgx_program_smem(P) + 1024);  // an SM's CTAs, by shared memory
+    int64_t per_sm = ((nlines + P->tb - 1) / P->tb + 151) / 152;
+    if (per_sm < 1) per_sm = 1;
+    if (per_sm > room) break;
+    int nt = (int)(PGX_MAX_THREADS_FFT / per_sm) / 32 * 32;
+    if (nt < 96 || P->tb * N > 16 * nt) continue;
+    const int most = (P->tb / 2 * N + 64) / 32 * 32;
+    if (nt > most) nt = most;
+    if (nt > 384) nt = 384;
+    // a warp a chain (four of two lines) while that costs no residency
+    if (warp_chains && nt < 128 && 128 * per_sm <= PGX_MAX_THREADS_FFT) nt = 128;
+    P->nthreads = nt;
+    return;
+  }
+  P->tb = N > 1024 ? 2 : 2048 / N / 2 * 2;
+  if (P->tb < 4 && N <= 1024) P->tb = 4;
+  if (P->tb > 16) P->tb = 16;
+  while (P->tb > 2 && 3 * (pgx_program_smem(P) + 1024) > smem_optin_max()) P->tb -= 2;
+  P->nthreads = (P->tb * N / 16 + 31) / 32 * 32;
+  if (P->nthreads < 64) P->nthreads = 64;
+  if (P->nthreads > 256) P->nthreads = 256;
+}
+
 // Lines per CTA and CTA size for a single-instance pass.
 void pick_tile(pgx_program* P, int nlines, int maxlen, int nbuf, int fft_n) {
   P->lcap = round_odd(maxlen + 1);
-  // FFT buffers: 2 buffers x stride complex per line pair (see pgx_fft_stride)
-  int64_t stride = fft_n > 1 ? (((fft_n - 1) & 1) == 0 ? fft_n - 1 : 2 * (fft_n - 1)) : 0;
-  int64_t per_line = (int64_t)8 * nbuf * P->lcap + 16 * stride + 8;
-  int64_t budget = smem_optin_max() - 4096;
+  // Sequential chain sweeps with few lines in the launch (fewer chains than ~64 per SM)
+  // run one warp per (line, parity) chain with a warp-parallel scan.
+  bool chains = false;
+  for (int o = 0; o < P->nops; ++o) {
+    const int code = P->ops[o].code;
+    chains |= code == PGX_OP_TDMA2 || code == PGX_OP_FDMA || code == PGX_OP_FDMA_T || code == PGX_OP_POISSON ||
+              code == PGX_OP_POISSON_T;
+  }
+  const bool warp_chains = chains && 2 * (int64_t)nlines < 152 * 64;
+  if (warp_chains) {
+    for (int o = 0; o < P->nops; ++o) {
+      pgx_op& op = P->ops[o];
+      if (op.code == PGX_OP_TDMA2 || op.code == PGX_OP_FDMA || op.code == PGX_OP_FDMA_T ||
+          op.code == PGX_OP_POISSON || op.code == PGX_OP_POISSON_T)
+        op.k = (int16_t)(op.k | PGX_CHAIN_WARP);
+    }
+  }
+  if (fft_n > 1) {
+    pick_fft_tile(P, nlines, warp_chains);
+    return;
+  }
+  const int64_t per_line = (int64_t)8 * nbuf * P->lcap + 8;
+  const int64_t budget = smem_optin_max() - 4096;
   int tbmax = (int)(budget / per_line);
   if (tbmax < 1) tbmax = 1;
   int tb = (nlines + 151) / 152;
-  if (fft_n > 1 && tb < 2) tb = 2;
   if (tb > 32) tb = 32;
   if (tb > tbmax) tb = tbmax;
   if (tb < 1) tb = 1;
@@ -424,21 +489,7 @@ void pick_tile(pgx_program* P, int nlines, int maxlen, int nbuf, int fft_n) {
   if (nt < 64) nt = 64;
   if (nt > 512) nt = 512;
   P->nthreads = nt;
-  // Sequential chain sweeps with few lines in the launch (fewer chains than ~64 per SM)
-  // run one warp per (line, parity) chain with a warp-parallel scan.
-  bool chains = false;
-  for (int o = 0; o < P->nops; ++o) {
-    const int code = P->ops[o].code;
-    chains |= code == PGX_OP_TDMA2 || code == PGX_OP_FDMA || code == PGX_OP_FDMA_T || code == PGX_OP_POISSON ||
-              code == PGX_OP_POISSON_T;
-  }
-  if (chains && 2 * (int64_t)nlines < 152 * 64) {
-    for (int o = 0; o < P->nops; ++o) {
-      pgx_op& op = P->ops[o];
-      if (op.code == PGX_OP_TDMA2 || op.code == PGX_OP_FDMA || op.code == PGX_OP_FDMA_T ||
-          op.code == PGX_OP_POISSON || op.code == PGX_OP_POISSON_T)
-        op.k = (int16_t)(op.k | PGX_CHAIN_WARP);
-    }
+  if (warp_chains) {
     int wt = 64 * tb;  // two chains (parities) per line, one warp each
     P->nthreads = wt < 256 ? 256 : (wt > PGX_MAX_THREADS ? PGX_MAX_THREADS : wt);
   }
