@@ -294,6 +294,24 @@ int pgx_stencil_from_chebyshev_t(const pgx_stencil_plan* plan,
                                  double* out, int64_t out_s0, int64_t out_s1,
                                  int32_t nlines, int32_t axis, void* stream);
 
+/* The compositions that pypde's transforms and gradients are made of, each one pass instead of two, and their
+ * transposes (transpose != 0: input and output lengths swap), for reverse mode:
+ *   values        backward_fft (chebyshev.py:268-285): S v, zero-padded to n >= N points (zero_pad,
+ *                 bases/utils.py:88-109), Chebyshev backward transform of n points;  N-2 -> n
+ *   coefficients  forward_fft (chebyshev.py:241-266): n <= N points zero-padded to N, Chebyshev forward
+ *                 transform, S^T, (S^T S)^-1;  n -> N-2
+ *   derivative    derivative (chebyshev.py:347-363): D^count S v;  N-2 -> N */
+int pgx_stencil_one_pass(int32_t n, int32_t nlines);  /* 0: lines of n points are faster as two passes */
+int pgx_stencil_values(const pgx_stencil_plan* plan, const double* in, int64_t in_s0, int64_t in_s1,
+                       double* out, int64_t out_s0, int64_t out_s1, int32_t n, int32_t nlines, int32_t axis,
+                       int32_t transpose, void* stream);
+int pgx_stencil_coefficients(const pgx_stencil_plan* plan, const double* in, int64_t in_s0, int64_t in_s1,
+                             double* out, int64_t out_s0, int64_t out_s1, int32_t n, int32_t nlines,
+                             int32_t axis, int32_t transpose, void* stream);
+int pgx_stencil_derivative(const pgx_stencil_plan* plan, const double* in, int64_t in_s0, int64_t in_s1,
+                           double* out, int64_t out_s0, int64_t out_s1, int32_t count, int32_t nlines,
+                           int32_t axis, int32_t transpose, void* stream);
+
 /* Offset-k tridiagonal solve, k = 2 (tdma.solve_tdma_1d/_2d, tdma.f90:2-107,
  * called from tdma.py:92-100).  a (n-2), b (n), c (n-2) are HOST arrays. */
 typedef struct pgx_tdma_plan pgx_tdma_plan;

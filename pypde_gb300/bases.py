@@ -216,14 +216,55 @@ class GalerkinChebyshev(MetaBase):
         f = to_dev(f)
         if bc is not None:
             f = f - self.eval_inhomogeneous(bc)
+        if self._one_pass_transform(f, self.N):
+            return self._coefficients(f)
         return self.from_chebyshev(self.family.forward_fft(f))
 
     def backward_fft(self, c, bc=None):
         """Galerkin coefficients -> physical (chebyshev.py:268-285)."""
+        c = to_dev(c)
+        if bc is None and self._one_pass_transform(c, self.N):
+            return self._values(c, self.family)
         u = self.to_chebyshev(c)
         if bc is not None:
             u = u + self.bc.to_chebyshev(bc)
         return self.family.backward_fft(u)
+
+    # The stencil and the Chebyshev operator beside it run as one pass (pgx_stencil_values and its
+    # neighbours), forward and transposed, unless a subclass maps to or from Chebyshev in its own way or
+    # the transform's form makes two passes the faster ones (pgx_stencil_one_pass).
+    def _one_pass(self):
+        cls, g = type(self), GalerkinChebyshev
+        return (cls.to_chebyshev is g.to_chebyshev and cls.from_chebyshev is g.from_chebyshev
+                and type(self.family) is Chebyshev)
+
+    def _one_pass_transform(self, x, n):
+        return (self._one_pass() and x.dim() in (1, 2)
+                and _lib.lib().pgx_stencil_one_pass(n, x.shape[1] if x.dim() == 2 else 1))
+
+    def _composed(self, x, fn, n_out, arg, transpose):
+        out = empty_like_axis(x, 0, n_out)
+        p, s0, s1, _, nl = geom(x, 0)
+        q, t0, t1, _, _ = geom(out, 0)
+        _lib.check(getattr(_lib.lib(), fn)(self._plan.h, p, s0, s1, q, t0, t1, arg, nl, 0, transpose, stream()), fn)
+        return out
+
+    def _coefficients(self, f):
+        """forward_fft of lines of at most N points (zero-padded to N)."""
+        n, N = f.shape[0], self.N
+        if n > N:
+            raise ValueError("input or output longer than the base")
+        return linear(f, lambda x: self._composed(x, "pgx_stencil_coefficients", N - 2, n, 0),
+                      lambda g: self._composed(g, "pgx_stencil_coefficients", n, n, 1))
+
+    def _values(self, c, family):
+        """Coefficients -> values on the points of ``family``, a Chebyshev base of at least N points."""
+        M, n = self.M, family.N
+        assert c.shape[0] == M, "{} {}".format(c.shape[0], M)
+        if n < self.N:
+            raise ValueError("input or output longer than the base")
+        return linear(c, lambda x: self._composed(x, "pgx_stencil_values", n, n, 0),
+                      lambda g: self._composed(g, "pgx_stencil_values", M, n, 1))
 
     def _stencil_op(self, x, fn, n_in, n_out):
         if x.shape[0] != n_in:
@@ -253,7 +294,14 @@ class GalerkinChebyshev(MetaBase):
 
     def derivative(self, vhat, deriv, out_cheby=True):
         """Derivative of Galerkin coefficients, Chebyshev output (chebyshev.py:347-363)."""
-        duhat = self.family.derivative(self.to_chebyshev(vhat), deriv)
+        if 0 < deriv < 1 << 15 and self._one_pass():
+            v = _along0(vhat)
+            M, N = self.M, self.N
+            assert v.shape[0] == M, "{} {}".format(v.shape[0], M)
+            duhat = linear(v, lambda x: self._composed(x, "pgx_stencil_derivative", N, deriv, 0),
+                           lambda g: self._composed(g, "pgx_stencil_derivative", M, deriv, 1))
+        else:
+            duhat = self.family.derivative(self.to_chebyshev(vhat), deriv)
         if out_cheby:
             return duhat
         return self.from_chebyshev(duhat)

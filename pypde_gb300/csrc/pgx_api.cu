@@ -808,6 +808,143 @@ extern "C" int pgx_stencil_from_chebyshev_t(const pgx_stencil_plan* p, const dou
   return pgx_run(&P, &I, stream);
 }
 
+// ------------------------------------------------------- composed passes
+// A transform and the stencil beside it as one pass: the field is read and written once and one launch is
+// issued where two passes took two, with an intermediate array between them.  The ops, their order and their
+// rounding are those of the separate passes.  Measured on GB300 along one axis of an N x N field, against those:
+// backward 9.0 us (14.4) at N = 65, 12.5 (18.8) at 257, 34.7 (44.8) at 1025; forward 11.8 (16.8), 17.5 (24.3), 85.8
+// (93.4); derivative 5.4 (8.9), 6.6 (10.4), 17.5 (28.2).
+//
+// The DCT of n points inside a composed pass: the op, its table and the program's FFT length.
+// Beside a mass solve short lines keep to the FFT where there is one: its pairs of lines give the chains warps on
+// every SM, which the dense form's tiles of eight do not (33 x 33: 11.4 us against 13.8).
+static int dct_op(pgx_program& P, pgx_instance& I, int at, int mat, int len, int n, int nlines, int mode) {
+  const double* tab = nullptr;
+  const bool solve = mode == PGX_DCT_FWD || mode == PGX_DCT_FWD_T;
+  const bool fft = solve ? pgx_fft_length_ok(n) : dct_use_fft(n, nlines);
+  const int rc = fft ? twiddles(n, &tab) : dense_dct(n, mode, &tab);
+  if (rc) return rc;
+  I.mat[mat] = tab;
+  if (fft) {
+    P.ops[at] = mk(PGX_OP_DCT, 0, -1, -1, mat, -1, mode);
+    P.fft_n = n;
+  } else {
+    P.ops[at] = mk(PGX_OP_DENSE, 0, -1, -1, mat, len, n <= DENSE_MMA_MAX_N ? PGX_DENSE_MMA : 0);
+  }
+  return PGX_OK;
+}
+// Its tile, by the rules of a transform alone: eight lines a CTA where the dense form runs on the tensor cores.
+static void composed_tile(pgx_program& P, int nlines, int n, bool dct) {
+  pick_tile(&P, nlines, n, 2, P.fft_n);
+  if (!dct || P.fft_n) return;
+  if (n <= DENSE_MMA_MAX_N) {
+    P.tb = 8;
+    const bool chains = P.nops > 3 && P.ops[P.nops - 2].code == PGX_OP_TDMA2;
+    P.nthreads = chains ? 64 * P.tb : 32 * ((n + 7) / 8);
+  }
+}
+static bool composed_args(const double* in, const double* out, int nlines, int axis) {
+  return in && out && nlines >= 0 && axis >= 0 && axis <= 1;
+}
+
+// Where the transform is a long dense contraction of many lines, its rows are split over CTAs (dense_tile), which
+// the ops beside it cannot be: two passes (460 lines of 132 points, forward: 24 us against 31 as one).
+extern "C" int pgx_stencil_one_pass(int32_t n, int32_t nlines) {
+  return nlines < 3 * 152 || n <= DENSE_MMA_MAX_N || pgx_fft_length_ok(n);
+}
+
+extern "C" int pgx_stencil_values(const pgx_stencil_plan* p, const double* in, int64_t in_s0, int64_t in_s1, double* out,
+                                  int64_t out_s0, int64_t out_s1, int32_t n, int32_t nlines, int32_t axis,
+                                  int32_t transpose, void* stream) {
+  if (!p) return PGX_E_PLAN;
+  if (!composed_args(in, out, nlines, axis) || n < p->N || n > PGX_LMAX - 8) return PGX_E_ARG;
+  pgx_program P;
+  pgx_instance I;
+  init_prog(P, I, axis);
+  I.len[0] = nlines;
+  I.len[1] = p->N - 2;
+  I.len[2] = n;
+  I.len[3] = p->N;
+  I.mat[0] = p->sub;
+  const int mode = transpose ? PGX_DCT_BWD_T : PGX_DCT_BWD;
+  set_axis_arr(I, 0, in, in_s0, in_s1, axis, transpose ? n : p->N - 2, nlines);
+  set_axis_arr(I, 1, out, out_s0, out_s1, axis, transpose ? p->N - 2 : n, nlines);
+  P.nops = 5;
+  int rc;
+  if (!transpose) {
+    P.ops[0] = mk(PGX_OP_LOAD, 0, -1, 0, -1, 1);
+    P.ops[1] = mk(PGX_OP_STENCIL, 0, -1, -1, 0);
+    P.ops[2] = mk(PGX_OP_SETLEN, 0, -1, -1, -1, 2);
+    rc = dct_op(P, I, 3, 1, 2, n, nlines, mode);
+  } else {
+    P.ops[0] = mk(PGX_OP_LOAD, 0, -1, 0, -1, 2);
+    rc = dct_op(P, I, 1, 1, 2, n, nlines, mode);
+    P.ops[2] = mk(PGX_OP_SETLEN, 0, -1, -1, -1, 3);
+    P.ops[3] = mk(PGX_OP_STENCIL_T, 0, -1, -1, 0);
+  }
+  if (rc) return rc;
+  P.ops[4] = mk(PGX_OP_STORE, 0, -1, 1);
+  composed_tile(P, nlines, n, true);
+  return pgx_run(&P, &I, stream);
+}
+
+extern "C" int pgx_stencil_coefficients(const pgx_stencil_plan* p, const double* in, int64_t in_s0, int64_t in_s1,
+                                        double* out, int64_t out_s0, int64_t out_s1, int32_t n, int32_t nlines, int32_t axis,
+                                        int32_t transpose, void* stream) {
+  if (!p) return PGX_E_PLAN;
+  if (!composed_args(in, out, nlines, axis) || n < 0 || n > p->N) return PGX_E_ARG;
+  pgx_program P;
+  pgx_instance I;
+  init_prog(P, I, axis);
+  I.len[0] = nlines;
+  I.len[1] = p->N;
+  I.len[2] = p->N - 2;
+  I.mat[0] = p->sub;
+  I.mat[1] = p->tdma;
+  set_axis_arr(I, 0, in, in_s0, in_s1, axis, transpose ? p->N - 2 : n, nlines);
+  set_axis_arr(I, 1, out, out_s0, out_s1, axis, transpose ? n : p->N - 2, nlines);
+  P.nops = 5;
+  int rc;
+  if (!transpose) {
+    P.ops[0] = mk(PGX_OP_LOAD, 0, -1, 0, -1, 1);
+    rc = dct_op(P, I, 1, 2, 1, p->N, nlines, PGX_DCT_FWD);
+    P.ops[2] = mk(PGX_OP_STENCIL_T, 0, -1, -1, 0);
+    P.ops[3] = mk(PGX_OP_TDMA2, 0, -1, -1, 1);
+  } else {
+    P.ops[0] = mk(PGX_OP_LOAD, 0, -1, 0, -1, 2);
+    P.ops[1] = mk(PGX_OP_TDMA2, 0, -1, -1, 1);
+    P.ops[2] = mk(PGX_OP_STENCIL, 0, -1, -1, 0);
+    rc = dct_op(P, I, 3, 2, 1, p->N, nlines, PGX_DCT_FWD_T);
+  }
+  if (rc) return rc;
+  P.ops[4] = mk(PGX_OP_STORE, 0, -1, 1);
+  composed_tile(P, nlines, p->N, true);
+  return pgx_run(&P, &I, stream);
+}
+
+extern "C" int pgx_stencil_derivative(const pgx_stencil_plan* p, const double* in, int64_t in_s0, int64_t in_s1,
+                                      double* out, int64_t out_s0, int64_t out_s1, int32_t count, int32_t nlines,
+                                      int32_t axis, int32_t transpose, void* stream) {
+  if (!p) return PGX_E_PLAN;
+  if (!composed_args(in, out, nlines, axis) || count < 0 || count > 32767) return PGX_E_ARG;
+  pgx_program P;
+  pgx_instance I;
+  init_prog(P, I, axis);
+  I.len[0] = nlines;
+  I.len[1] = p->N - 2;
+  I.len[2] = p->N;
+  I.mat[0] = p->sub;
+  set_axis_arr(I, 0, in, in_s0, in_s1, axis, transpose ? p->N : p->N - 2, nlines);
+  set_axis_arr(I, 1, out, out_s0, out_s1, axis, transpose ? p->N - 2 : p->N, nlines);
+  P.nops = 4;
+  P.ops[0] = mk(PGX_OP_LOAD, 0, -1, 0, -1, transpose ? 2 : 1);
+  P.ops[transpose ? 2 : 1] = mk(transpose ? PGX_OP_STENCIL_T : PGX_OP_STENCIL, 0, -1, -1, 0);
+  P.ops[transpose ? 1 : 2] = mk(transpose ? PGX_OP_DIFF_T : PGX_OP_DIFF, 0, -1, -1, -1, -1, count);
+  P.ops[3] = mk(PGX_OP_STORE, 0, -1, 1);
+  composed_tile(P, nlines, p->N, false);
+  return pgx_run(&P, &I, stream);
+}
+
 extern "C" int pgx_tdma_plan_create(const double* a, const double* b, const double* c, int32_t n, int32_t k,
                                     pgx_tdma_plan** plan) {
   if (!a || !b || !c || !plan || n < 3 || n > PGX_LMAX - 8 || k != 2) return PGX_E_ARG;

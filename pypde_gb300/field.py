@@ -9,7 +9,7 @@ import torch
 
 from . import _lib
 from ._dev import to_dev, DTYPE, device
-from .bases import MetaBase
+from .bases import Chebyshev, GalerkinChebyshev, MetaBase
 from .spectralspace import SpectralSpace, SpectralSpaceBC
 
 
@@ -39,10 +39,13 @@ def _values(coef_base, grid_base, c):
     """Coefficient lines of ``coef_base`` -> values on ``grid_base``'s points (axis 0).  A shorter
     coefficient base (the undealiased one) is not padded by a copy: the stencil maps its own
     coefficients to Chebyshev ones, and the backward DCT of the grid's length reads those and
-    zero-fills the rest of the line (the kernel's input length, like the fused passes' SETLEN).
+    zero-fills the rest of the line (one pass; the kernel's input length, like the fused passes' SETLEN).
     Zero-padding commutes with the Shen stencils, whose entries depend on the row index only."""
-    u = coef_base.to_chebyshev(c) if hasattr(coef_base, "to_chebyshev") else _as_lines(c)
     fam = getattr(grid_base, "family", grid_base)
+    if (isinstance(coef_base, GalerkinChebyshev) and type(fam) is Chebyshev
+            and coef_base._one_pass_transform(c, fam.N)):
+        return coef_base._values(c, fam)
+    u = coef_base.to_chebyshev(c) if hasattr(coef_base, "to_chebyshev") else _as_lines(c)
     return fam._dct(u, _lib.DCT_BWD)
 
 
