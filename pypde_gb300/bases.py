@@ -13,7 +13,7 @@ import scipy.sparse
 import torch
 
 from . import _lib
-from ._dev import empty_like_axis, geom, stream, to_dev
+from ._dev import geom, new_along, stream, to_dev
 from .autodiff import linear
 from .host import (dealias_size, gauss_lobatto, pseudoinverse_d2, stencil_matrix)
 
@@ -104,10 +104,9 @@ class Chebyshev(MetaBase):
         n_in = f.shape[0]
         if n_in > self.N or n_out > self.N:
             raise ValueError("input or output longer than the base")
-        out = empty_like_axis(f, 0, n_out)
         p, s0, s1, _, nl = geom(f, 0)
-        q, t0, t1, no, _ = geom(out, 0)
-        _lib.check(_lib.lib().pgx_dct1(p, s0, s1, n_in, q, t0, t1, no, self.N, nl, 0, mode, stream()), "dct1")
+        out, q, t0, t1 = new_along(f, 0, n_out)
+        _lib.check(_lib.lib().pgx_dct1(p, s0, s1, n_in, q, t0, t1, n_out, self.N, nl, 0, mode, stream()), "dct1")
         return out
 
     def _dct(self, f, mode, n_out=None):
@@ -149,9 +148,8 @@ class Chebyshev(MetaBase):
 
     @staticmethod
     def _diff(f, deriv, fn):
-        out = empty_like_axis(f, 0, f.shape[0])
         p, s0, s1, n, nl = geom(f, 0)
-        q, t0, t1, _, _ = geom(out, 0)
+        out, q, t0, t1 = new_along(f, 0, n)
         _lib.check(getattr(_lib.lib(), fn)(p, s0, s1, q, t0, t1, n, nl, 0, deriv, stream()), fn)
         return out
 
@@ -243,9 +241,8 @@ class GalerkinChebyshev(MetaBase):
                 and _lib.lib().pgx_stencil_one_pass(n, x.shape[1] if x.dim() == 2 else 1))
 
     def _composed(self, x, fn, n_out, arg, transpose):
-        out = empty_like_axis(x, 0, n_out)
         p, s0, s1, _, nl = geom(x, 0)
-        q, t0, t1, _, _ = geom(out, 0)
+        out, q, t0, t1 = new_along(x, 0, n_out)
         _lib.check(getattr(_lib.lib(), fn)(self._plan.h, p, s0, s1, q, t0, t1, arg, nl, 0, transpose, stream()), fn)
         return out
 
@@ -269,9 +266,8 @@ class GalerkinChebyshev(MetaBase):
     def _stencil_op(self, x, fn, n_in, n_out):
         if x.shape[0] != n_in:
             raise ValueError("%s: expected %d points along the axis, got %d" % (fn, n_in, x.shape[0]))
-        out = empty_like_axis(x, 0, n_out)
         p, s0, s1, _, nl = geom(x, 0)
-        q, t0, t1, _, _ = geom(out, 0)
+        out, q, t0, t1 = new_along(x, 0, n_out)
         _lib.check(getattr(_lib.lib(), fn)(self._plan.h, p, s0, s1, q, t0, t1, nl, 0, stream()), fn)
         return out
 
@@ -403,9 +399,8 @@ class MatrixApply:
     def _apply(self, b, axis):
         if b.shape[axis] != self.cols:
             raise ValueError("Shape mismatch: N {:4d} | b.shape[axis] {:4d}".format(self.cols, b.shape[axis]))
-        out = empty_like_axis(b, axis, self.rows)
         p, s0, s1, _, nl = geom(b, axis)
-        q, t0, t1, _, _ = geom(out, axis)
+        out, q, t0, t1 = new_along(b, axis, self.rows)
         _lib.check(_lib.lib().pgx_matrix_apply(self.h, p, s0, s1, q, t0, t1, nl, axis, stream()), "matrix apply")
         return out
 
