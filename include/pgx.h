@@ -114,6 +114,9 @@ enum pgx_dct_mode { PGX_DCT_RAW = 0, PGX_DCT_FWD = 1, PGX_DCT_BWD = 2, PGX_DCT_F
  * warp per (line, parity) chain with a warp-parallel scan instead of one thread
  * per chain (for passes with few lines). */
 #define PGX_CHAIN_WARP 1
+/* op.k of FDMA / FDMA_T / POISSON / POISSON_T beside PGX_CHAIN_WARP: the scan's maps are in the table, behind the
+ * factors, where pgx_chain_pack writes them; the same values with fewer operations. */
+#define PGX_CHAIN_SCAN 2
 /* op.k of DENSE: PGX_DENSE_MMA runs the contraction on the FP64 tensor cores (DMMA,
  * 8 x 8 x 4 tiles: rows x lines x columns) instead of one FMA chain per output. */
 #define PGX_DENSE_MMA 2
@@ -376,6 +379,13 @@ int pgx_matrix_plan_is_banded(const pgx_matrix_plan* plan);
  * matrix's digits (asynchronously on `stream`). */
 int64_t pgx_dense_doubles(int32_t rows, int32_t cols);
 int pgx_dense_pack(double* A, int32_t rows, int32_t cols, void* stream);
+
+/* A table for PGX_CHAIN_SCAN, in DEVICE memory: `tab` holds the factors, nlines systems of 4n doubles (FDMA: one
+ * system), at the start of a 16-byte aligned buffer of pgx_chain_doubles(n, nlines) doubles, and pgx_chain_pack
+ * fills the rest with the maps of the warp scan (asynchronously on `stream`).  A POISSON op's nlines are its
+ * instance's lines. */
+int64_t pgx_chain_doubles(int32_t n, int32_t nlines);
+int pgx_chain_pack(double* tab, int32_t n, int32_t nlines, void* stream);
 
 /* Device table of DCT ops for line programs built by the host: twiddle factors of
  * the DCT-I of n points (2(n-1) complex values exp(-2 pi i k / (2(n-1))), then the

@@ -18,6 +18,7 @@ OP = dict(LOAD=1, LOAD_ADD=2, LOAD_MUL=3, STORE=4, STORE_ADD=5, SCALE=6, AXPY=7,
           FDMA=19, POISSON=20, ZERO00=21, DIFF_T=22, FDMA_T=23, POISSON_T=24)
 DCT_RAW, DCT_FWD, DCT_BWD, DCT_FWD_T, DCT_BWD_T = 0, 1, 2, 3, 4
 CHAIN_WARP = 1  # op.k flag of the chain ops: one warp per chain (PGX_CHAIN_WARP)
+CHAIN_SCAN = 2  # op.k flag of the FDMA / POISSON ops beside it: scan maps in the table (PGX_CHAIN_SCAN)
 DENSE_TC = 4    # op.k flag of DENSE: contraction in digits on the FP16 tensor cores (PGX_DENSE_TC)
 DENSE_MMA = 2   # op.k flag of DENSE: contraction on the FP64 tensor cores (PGX_DENSE_MMA)
 DCT_SLOT = 16   # op.k flag of DCT: the FFT in the slot's own lines and the spare (PGX_DCT_SLOT)
@@ -138,6 +139,8 @@ SIGNATURES = {
     "pgx_matrix_apply": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_int64,
                                         ctypes.c_void_p, ctypes.c_int64, ctypes.c_int64, ctypes.c_int32,
                                         ctypes.c_int32, ctypes.c_void_p]),
+    "pgx_chain_doubles": (ctypes.c_int64, [ctypes.c_int32, ctypes.c_int32]),
+    "pgx_chain_pack": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int32, ctypes.c_void_p]),
     "pgx_dense_doubles": (ctypes.c_int64, [ctypes.c_int32, ctypes.c_int32]),
     "pgx_dense_pack": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int32, ctypes.c_void_p]),
     "pgx_dct_table": (ctypes.c_int, [ctypes.c_int32, ctypes.c_void_p]),

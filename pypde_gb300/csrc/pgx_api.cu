@@ -27,6 +27,8 @@ int launch_persistent(const pgx_program* d_progs, int nprogs, const pgx_instance
                       const pgx_persist_item* d_items, int nitems, int32_t* d_counters, int ncounters,
                       int32_t* d_state, int ctas, int threads, int64_t smem, long long spin_limit, cudaStream_t s);
 int dense_pack(const double* d_A, int rows, int cols, void* d_packed, cudaStream_t s);
+int chain_map_doubles();
+int chain_pack(double* d_tab, int n, int nlines, cudaStream_t s);
 }
 
 static thread_local int g_last_cuda = 0;
@@ -254,6 +256,18 @@ extern "C" int pgx_dense_pack(double* A, int32_t rows, int32_t cols, void* strea
   return e ? cuda_fail((cudaError_t)e) : PGX_OK;
 }
 
+// nlines systems of 4n factors, and the maps of their chains
+extern "C" int64_t pgx_chain_doubles(int32_t n, int32_t nlines) {
+  if (n < 1 || nlines < 1) return 0;
+  return (int64_t)nlines * (4 * (int64_t)n + pgx::chain_map_doubles());
+}
+
+extern "C" int pgx_chain_pack(double* tab, int32_t n, int32_t nlines, void* stream) {
+  if (!tab || ((uintptr_t)tab & 15) || n < 1 || n > PGX_LMAX || nlines < 1 || nlines > (1 << 26)) return PGX_E_ARG;
+  const int e = pgx::chain_pack(tab, n, nlines, (cudaStream_t)stream);
+  return e ? cuda_fail((cudaError_t)e) : PGX_OK;
+}
+
 namespace {
 std::mutex g_mu;
 
@@ -277,6 +291,22 @@ int upload_dense(const std::vector<double>& h, int rows, int cols, double** d) {
   if (e != cudaSuccess) return cuda_fail(e);
   e = cudaMemcpy(p, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice);
   int rc = e == cudaSuccess ? pgx_dense_pack((double*)p, rows, cols, nullptr) : cuda_fail(e);
+  if (!rc && (e = cudaStreamSynchronize(nullptr)) != cudaSuccess) rc = cuda_fail(e);
+  if (rc) {
+    cudaFree(p);
+    return rc;
+  }
+  *d = (double*)p;
+  return PGX_OK;
+}
+
+// FDMA or POISSON factors with the maps of PGX_CHAIN_SCAN behind them.
+int upload_chain(const std::vector<double>& h, int n, int nlines, double** d) {
+  void* p = nullptr;
+  cudaError_t e = cudaMalloc(&p, (size_t)pgx_chain_doubles(n, nlines) * sizeof(double));
+  if (e != cudaSuccess) return cuda_fail(e);
+  e = cudaMemcpy(p, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice);
+  int rc = e == cudaSuccess ? pgx_chain_pack((double*)p, n, nlines, nullptr) : cuda_fail(e);
   if (!rc && (e = cudaStreamSynchronize(nullptr)) != cudaSuccess) rc = cuda_fail(e);
   if (rc) {
     cudaFree(p);
@@ -468,7 +498,7 @@ void pick_tile(pgx_program* P, int nlines, int maxlen, int nbuf, int fft_n) {
       pgx_op& op = P->ops[o];
       if (op.code == PGX_OP_TDMA2 || op.code == PGX_OP_FDMA || op.code == PGX_OP_FDMA_T ||
           op.code == PGX_OP_POISSON || op.code == PGX_OP_POISSON_T)
-        op.k = (int16_t)(op.k | PGX_CHAIN_WARP);
+        op.k = (int16_t)(op.k | PGX_CHAIN_WARP | (op.code == PGX_OP_TDMA2 ? 0 : PGX_CHAIN_SCAN));
     }
   }
   if (fft_n > 1) {
@@ -992,7 +1022,7 @@ extern "C" int pgx_tdma_solve(const pgx_tdma_plan* p, const double* d, int64_t d
 // ------------------------------------------------------------------ FDMA
 struct pgx_fdma_plan {
   int n;
-  double* tab;  // [l | dinv | u1 dinv | u2 dinv]
+  double* tab;  // [l | dinv | u1 dinv | u2 dinv], scan maps
 };
 
 static void fdma_tab(const double* l, const double* d, const double* u1, const double* u2, int n,
@@ -1014,7 +1044,7 @@ extern "C" int pgx_fdma_plan_create(const double* l, const double* d, const doub
   fdma_tab(l, d, u1, u2, n, tab, 0);
   pgx_fdma_plan* p = new pgx_fdma_plan();
   p->n = n;
-  int rc = upload(tab, &p->tab);
+  int rc = upload_chain(tab, n, 1, &p->tab);
   if (rc) {
     delete p;
     return rc;
@@ -1069,7 +1099,7 @@ static int fdma_solve_op(int code, const pgx_fdma_plan* p, double* x, int64_t s0
 // ---------------------------------------------------------------- Poisson
 struct pgx_poisson_plan {
   int n, m;
-  double* tab;  // m lines x [l | dinv | u1 dinv | u2 dinv] (n each)
+  double* tab;  // m lines x [l | dinv | u1 dinv | u2 dinv] (n each), then their scan maps
 };
 
 // LU sweep of the four diagonals of an n x n band (init_fdma's recurrence).
@@ -1118,7 +1148,7 @@ extern "C" int pgx_poisson_plan_create(const double* A, const double* C, const d
   pgx_poisson_plan* p = new pgx_poisson_plan();
   p->n = n;
   p->m = m;
-  int rc = upload(tab, &p->tab);
+  int rc = upload_chain(tab, n, m, &p->tab);
   if (rc) {
     delete p;
     return rc;

@@ -660,6 +660,7 @@ __device__ __forceinline__ int nslot_of(const pgx_op& op) { return op.b > 1 ? op
 // its exact incoming state.  The work grows ~3x, the dependent path shrinks from
 // n/2 steps to ~n/32 + 5 combine levels.
 constexpr unsigned FULLMASK = 0xffffffffu;
+__device__ __forceinline__ void prefetch_l1(const double* a) { asm volatile("prefetch.L1 [%0];" ::"l"(a)); }
 
 // y_q = b(q) + a(q) y_{q-1} for q = 0..m-1 (recurrence order), y_{-1} = 0; put(q, y).
 template <class FA, class FB, class FP>
@@ -697,7 +698,7 @@ __device__ __forceinline__ void warp_rec2(int m, int lane, FA1 a1, FA2 a2, FB b,
   double m00 = 1.0, m01 = 0.0, m10 = 0.0, m11 = 1.0, c0 = 0.0, c1 = 0.0;
   for (int q = q0; q < q1; ++q) {
     const double x1 = a1(q), x2 = a2(q);
-    const double n00 = fma(x2, m10, x1 * m00), n01 = fma(x2, m11, x1 * m01);
+    const double n00 = fma(x2, m10, __dmul_rn(x1, m00)), n01 = fma(x2, m11, __dmul_rn(x1, m01));
     const double nc0 = fma(x2, c1, fma(x1, c0, b(q)));
     m10 = m00;
     m11 = m01;
@@ -731,6 +732,158 @@ __device__ __forceinline__ void warp_rec2(int m, int lane, FA1 a1, FA2 a2, FB b,
     y1 = y;
     put(q, y);
   }
+}
+
+// The scans with the segment maps from the table (PGX_CHAIN_SCAN).  The maps depend on the factors only, and
+// composing them is most of the two functions above: of the 83 FP64 instructions of a 63-point solve's two sweeps,
+// 66 cycles of an SM quarter each, 33 are left, of 511 points 190 and 80.  The values are the same to the bit: the
+// maps are those that the functions above compose (chain_pack), and the states meet them in the same order.
+// (__dmul_rn: in a peeled step, whose map holds a 1, the compiler would be free to fuse the other product instead.)
+// Maps of a chain: kChainMaps doubles, 5 levels x 32 lanes of the first-order sweep, then 5 x 2 rows x 32 lanes x 2
+// of the second-order one (a warp's loads of a level are contiguous).
+constexpr int kChainMaps = 160 + 640;
+template <class FA, class FB, class FP>
+__device__ __forceinline__ void scan_rec1(int m, int lane, const double* maps, FA a, FB b, FP put) {
+  const int C = (m + 31) >> 5;
+  const int q0 = min(lane * C, m), q1 = min(q0 + C, m);
+  double B = 0.0;
+  for (int q = q0; q < q1; ++q) B = fma(a(q), B, b(q));
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    const double A = __ldg(maps + 32 * k + lane);
+    const double Bp = __shfl_up_sync(FULLMASK, B, 1 << k);
+    if (lane >= 1 << k) B = fma(A, Bp, B);
+  }
+  double y = __shfl_up_sync(FULLMASK, B, 1);
+  if (lane == 0) y = 0.0;
+  for (int q = q0; q < q1; ++q) {
+    y = fma(a(q), y, b(q));
+    put(q, y);
+  }
+}
+// first(q): b(q) in the first walk, later(q): in the second (what first has stored, or the same again)
+template <class FA1, class FA2, class FB, class FL, class FP>
+__device__ __forceinline__ void scan_rec2(int m, int lane, const double* maps, FA1 a1, FA2 a2, FB first, FL later,
+                                          FP put) {
+  const int C = (m + 31) >> 5;
+  const int q0 = min(lane * C, m), q1 = min(q0 + C, m);
+  const double2* M = reinterpret_cast<const double2*>(maps);
+  double c0 = 0.0, c1 = 0.0;
+  for (int q = q0; q < q1; ++q) {
+    const double nc0 = fma(a2(q), c1, fma(a1(q), c0, first(q)));
+    c1 = c0;
+    c0 = nc0;
+  }
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    const double2 r0 = __ldg(M + 64 * k + lane), r1 = __ldg(M + 64 * k + 32 + lane);
+    const double pc0 = __shfl_up_sync(FULLMASK, c0, 1 << k), pc1 = __shfl_up_sync(FULLMASK, c1, 1 << k);
+    if (lane >= 1 << k) {
+      c0 = fma(r0.y, pc1, fma(r0.x, pc0, c0));
+      c1 = fma(r1.y, pc1, fma(r1.x, pc0, c1));
+    }
+  }
+  double y1 = __shfl_up_sync(FULLMASK, c0, 1), y2 = __shfl_up_sync(FULLMASK, c1, 1);
+  if (lane == 0) y1 = y2 = 0.0;
+  for (int q = q0; q < q1; ++q) {
+    const double y = fma(a2(q), y2, fma(a1(q), y1, later(q)));
+    y2 = y1;
+    y1 = y;
+    put(q, y);
+  }
+}
+
+// The coefficients of an FDMA chain's four sweeps, in recurrence order (see fdma_chain and fdma_t_chain).
+struct FdmaChain {
+  const double* tab;  // [l | dinv | u1 | u2]
+  int n, p, m;
+  __device__ __forceinline__ FdmaChain(const double* t, int n_, int p_) : tab(t), n(n_), p(p_), m((n_ - p_ + 1) >> 1) {}
+  __device__ __forceinline__ int up(int q) const { return p + 2 * q; }
+  __device__ __forceinline__ int down(int q) const { return p + 2 * (m - 1 - q); }
+  __device__ __forceinline__ double dinv(int i) const { return __ldg(tab + n + i); }
+  __device__ __forceinline__ double l(int q) const { return -__ldg(tab + up(q)); }
+  __device__ __forceinline__ double u1(int q) const { return -__ldg(tab + 2 * n + down(q)); }
+  __device__ __forceinline__ double u2(int q) const { return -__ldg(tab + 3 * n + down(q)); }
+  __device__ __forceinline__ double tu1(int q) const { return up(q) >= 2 ? -__ldg(tab + 2 * n + up(q) - 2) : 0.0; }
+  __device__ __forceinline__ double tu2(int q) const { return up(q) >= 4 ? -__ldg(tab + 3 * n + up(q) - 4) : 0.0; }
+  __device__ __forceinline__ double tl(int q) const { return down(q) + 2 < n ? -__ldg(tab + down(q) + 2) : 0.0; }
+};
+
+// `maps`: this chain's, of this direction.  One warp asks for all it will read at once.
+__device__ __forceinline__ void fdma_chain_scan(double* x, const double* tab, const double* maps, int n, int p,
+                                                int lane, bool transpose) {
+  const FdmaChain f(tab, n, p);
+  for (int i = 16 * lane; i < kChainMaps; i += 512) prefetch_l1(maps + i);
+  for (int i = 16 * lane; i < 4 * n; i += 512) prefetch_l1(tab + i);
+  if (!transpose) {
+    scan_rec1(f.m, lane, maps, [&](int q) { return f.l(q); }, [&](int q) { return x[f.up(q)]; },
+              [&](int q, double y) { x[f.up(q)] = y; });
+    __syncwarp();
+    scan_rec2(f.m, lane, maps + 160, [&](int q) { return f.u1(q); }, [&](int q) { return f.u2(q); },
+              [&](int q) { const int i = f.down(q); return x[i] *= f.dinv(i); }, [&](int q) { return x[f.down(q)]; },
+              [&](int q, double y) { x[f.down(q)] = y; });
+  } else {
+    scan_rec2(f.m, lane, maps + 160, [&](int q) { return f.tu1(q); }, [&](int q) { return f.tu2(q); },
+              [&](int q) { return x[f.up(q)]; }, [&](int q) { return x[f.up(q)]; },
+              [&](int q, double y) { const int i = f.up(q); x[i] = y * f.dinv(i); });
+    __syncwarp();
+    scan_rec1(f.m, lane, maps, [&](int q) { return f.tl(q); }, [&](int q) { return x[f.down(q)]; },
+              [&](int q, double y) { x[f.down(q)] = y; });
+  }
+}
+
+// The maps of every chain (pgx_chain_pack): after the nlines x 4n factors, per line and parity, the solve's and then
+// the transposed solve's, kChainMaps each.  A warp a chain; the compositions of warp_rec1 and warp_rec2.
+template <class FA>
+__device__ __forceinline__ void pack_maps1(int m, int lane, FA a, double* out) {
+  const int C = (m + 31) >> 5;
+  const int q0 = min(lane * C, m), q1 = min(q0 + C, m);
+  double A = 1.0;
+  for (int q = q0; q < q1; ++q) A *= a(q);
+  for (int k = 0; k < 5; ++k) {
+    out[32 * k + lane] = A;
+    const double Ap = __shfl_up_sync(FULLMASK, A, 1 << k);
+    if (lane >= 1 << k) A *= Ap;
+  }
+}
+template <class FA1, class FA2>
+__device__ __forceinline__ void pack_maps2(int m, int lane, FA1 a1, FA2 a2, double2* out) {
+  const int C = (m + 31) >> 5;
+  const int q0 = min(lane * C, m), q1 = min(q0 + C, m);
+  double m00 = 1.0, m01 = 0.0, m10 = 0.0, m11 = 1.0;
+  for (int q = q0; q < q1; ++q) {
+    const double x1 = a1(q), x2 = a2(q);
+    const double n00 = fma(x2, m10, __dmul_rn(x1, m00)), n01 = fma(x2, m11, __dmul_rn(x1, m01));
+    m10 = m00;
+    m11 = m01;
+    m00 = n00;
+    m01 = n01;
+  }
+  for (int k = 0; k < 5; ++k) {
+    out[64 * k + lane] = make_double2(m00, m01);
+    out[64 * k + 32 + lane] = make_double2(m10, m11);
+    const double p00 = __shfl_up_sync(FULLMASK, m00, 1 << k), p01 = __shfl_up_sync(FULLMASK, m01, 1 << k);
+    const double p10 = __shfl_up_sync(FULLMASK, m10, 1 << k), p11 = __shfl_up_sync(FULLMASK, m11, 1 << k);
+    if (lane >= 1 << k) {
+      const double r00 = fma(m01, p10, m00 * p00), r01 = fma(m01, p11, m00 * p01);
+      const double r10 = fma(m11, p10, m10 * p00), r11 = fma(m11, p11, m10 * p01);
+      m00 = r00;
+      m01 = r01;
+      m10 = r10;
+      m11 = r11;
+    }
+  }
+}
+__global__ void chain_pack_maps(const double* __restrict__ tab, double* __restrict__ maps, int n, int nlines) {
+  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (w >= 2 * nlines) return;  // a whole warp
+  const FdmaChain f(tab + (size_t)(w >> 1) * 4 * n, n, w & 1);
+  double* out = maps + (size_t)w * 2 * kChainMaps;
+  pack_maps1(f.m, lane, [&](int q) { return f.l(q); }, out);
+  pack_maps2(f.m, lane, [&](int q) { return f.u1(q); }, [&](int q) { return f.u2(q); }, (double2*)(out + 160));
+  out += kChainMaps;
+  pack_maps1(f.m, lane, [&](int q) { return f.tl(q); }, out);
+  pack_maps2(f.m, lane, [&](int q) { return f.tu1(q); }, [&](int q) { return f.tu2(q); }, (double2*)(out + 160));
 }
 
 // The chain of parity p of an n-point line, x[p + 2k], k < m = (n - p + 1) / 2.
@@ -974,7 +1127,6 @@ __device__ void op_diff_t(Ctx& c, const pgx_op& op) {
 // so they would come from L2 at every step.  Each step therefore asks L1 for the factors
 // PF elements ahead (in-bounds addresses only; a prefetch is a hint and changes no result).
 constexpr int PF = 32;
-__device__ __forceinline__ void prefetch_l1(const double* a) { asm volatile("prefetch.L1 [%0];" ::"l"(a)); }
 
 __device__ __forceinline__ void fdma_chain(double* x, const double* tab, int n, int p) {
   const double* l = tab;
@@ -1058,8 +1210,15 @@ __device__ void op_fdma(Ctx& c, const pgx_op& op, const pgx_instance& I, bool pe
       const int line = c_l0 + t;
       if (p >= n || line >= c_nlines) continue;
       const double* tab = I.mat[op.mat + (per_line ? 0 : s)];
-      if (per_line) tab += (size_t)line * 4 * n;
       double* x = slot_ptr(c, op.a + s) + t * c_lcap;
+      if (op.k & PGX_CHAIN_SCAN) {
+        const int sys = per_line ? line : 0;
+        const double* maps = tab + (size_t)(per_line ? c_nlines : 1) * 4 * n +
+                             (size_t)(4 * sys + 2 * p + (transpose ? 1 : 0)) * kChainMaps;
+        fdma_chain_scan(x, tab + (size_t)sys * 4 * n, maps, n, p, lane, transpose);
+        continue;
+      }
+      if (per_line) tab += (size_t)line * 4 * n;
       if (transpose) fdma_t_chain_warp(x, tab, n, p, lane);
       else fdma_chain_warp(x, tab, n, p, lane);
     }
@@ -2731,6 +2890,11 @@ int launch_batched(const pgx_program* P0, const pgx_instance* d_insts, const int
   return (int)cudaGetLastError();
 }
 
+int chain_map_doubles() { return 4 * kChainMaps; }  // a line's: two parities, two directions
+int chain_pack(double* d_tab, int n, int nlines, cudaStream_t s) {
+  chain_pack_maps<<<(2 * nlines + 3) / 4, 128, 0, s>>>(d_tab, d_tab + (size_t)nlines * 4 * n, n, nlines);
+  return (int)cudaGetLastError();
+}
 int dense_pack(const double* d_A, int rows, int cols, void* d_packed, cudaStream_t s) {
   const int rt = (rows + 15) / 16, kt = (cols + 15) / 16;
   uint4* digits = (uint4*)d_packed;

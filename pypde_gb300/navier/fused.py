@@ -621,12 +621,34 @@ def dense_dev(A):
     return buf
 
 
+def chain_dev(tab, n):
+    """The factors of one four-diagonal system of n unknowns, or of one a line, on the device with their scan
+    maps behind them (pgx_chain_pack)."""
+    lines = tab.size // (4 * n)
+    L = _lib.lib()
+    buf = torch.empty(L.pgx_chain_doubles(n, lines), dtype=DTYPE, device=device())
+    buf[:tab.size].copy_(torch.from_numpy(np.ascontiguousarray(tab)).reshape(-1))
+    _lib.check(L.pgx_chain_pack(buf.data_ptr(), n, lines, stream()), "chain pack")
+    return buf
+
+
 DENSE_TABLES = ("Hy", "Qy", "HyT", "QyT")
+CHAIN_TABLES = ("Ax_U", "Ax_T", "Ay_U", "Ay_T")
 
 
 def tables_dev(host):
-    """Host operator tables on the device (the dense ones with their digits)."""
-    return {k: dense_dev(v) if k in DENSE_TABLES else to_dev(v) for k, v in host.items()}
+    """Host operator tables on the device (the dense ones with their digits, the banded solves with their maps)."""
+    t = {}
+    for k, v in host.items():
+        if k in DENSE_TABLES:
+            t[k] = dense_dev(v)
+        elif k in CHAIN_TABLES:
+            t[k] = chain_dev(v, v.size // 4)
+        elif k == "Pois":  # systems along x, as long as the implicit x-operators
+            t[k] = chain_dev(v, host["Ax_U"].size // 4)
+        else:
+            t[k] = to_dev(v)
+    return t
 
 
 _DENSE_DCT_CACHE = {}
@@ -671,6 +693,7 @@ def host_tables(N, M, tk, dt, nu, kappa, scale, fd, adjoint=False):
     t["Ay_U"] = _fdma_table(By @ Sy - lu / sz ** 2 * Iy @ Sy)
     t["Ay_T"] = _fdma_table(By @ Sy - lt / sz ** 2 * Iy @ Sy)
     t["Pois"] = _poisson_table(np.asarray(fd["Ax"]), np.asarray(fd["Cx"]), np.real(fd["wy"]))
+    assert t["Pois"].size == 4 * (N - 2) * (M - 2)  # a system a line of the pass (the maps follow the last one)
     Hy, Qy = np.real(np.asarray(fd["Hy"])), np.real(np.asarray(fd["Qy"]))
     t["Hy"] = np.ascontiguousarray(Hy)
     t["Qy"] = np.ascontiguousarray(Qy)
@@ -786,7 +809,7 @@ class _Instance:
                                                       ak, bk, ck, bt)[1])
                 hs = host_tables(N, M, ns.T.xs[0].id, ns.dt * ak * bt, ns.nu, ns.kappa, ns.scale,
                                  ns.solver_P._fd)
-                self.stage_tables.append({k: to_dev(hs[k]) for k in ("Ax_U", "Ax_T", "Ay_U", "Ay_T")})
+                self.stage_tables.append(tables_dev({k: hs[k] for k in CHAIN_TABLES}))
                 cur, old = ("A", "A") if st == 0 else (("B", "A") if st == 1 else ("A", "B"))
                 self.stage_arrays.append({"UXC": "UX_" + cur, "UZC": "UZ_" + cur, "UXO": "UX_" + old,
                                           "UZO": "UZ_" + old})
@@ -1062,7 +1085,8 @@ def launch_program(prog, key, tb, nt, wc=False, sd=False, dm=False, tc=False):
     for i, o in enumerate(ops):
         P.ops[i] = o
         if wc and o.code in _CHAIN_CODES:
-            P.ops[i].k = o.k | _lib.CHAIN_WARP
+            scan = 0 if o.code == _lib.OP["TDMA2"] else _lib.CHAIN_SCAN  # (every table has its maps: chain_dev)
+            P.ops[i].k = o.k | _lib.CHAIN_WARP | scan
         if in_slot and o.code == _lib.OP["DCT"]:
             P.ops[i].k = o.k | _lib.DCT_SLOT
         if tc and o.code == _lib.OP["DENSE"]:  # every dense table carries its digits (dense_dev)
