@@ -526,12 +526,13 @@ void pick_tile(pgx_program* P, int nlines, int maxlen, int nbuf, int fft_n) {
 }
 
 // A LOAD, DENSE, STORE pass on the tensor cores, where that pays: an instruction takes eight lines whether they
-// are there or not, so a launch needs a few an SM to fill them (511 lines of 257 points 31 us against 72 us as
-// FP64 chains, 127 lines of 129 points 11 us against 8).  Eight lines a CTA (the launch splits the rows over
-// CTAs), a warp per row block up to eight.
+// are there or not, and the launch splits the rows over CTAs; the FP64 chains take one wave of lines after the
+// other, rows x columns each.  They lose from about 200 rows x waves on: 8 lines of 257 points 20 us against 35,
+// 129 lines of 129 points 13.8 against 11.1, 193 such lines 13.6 against 15.3, 400 lines of 385 points 39 against
+// 128.  Eight lines a CTA, a warp per row block up to eight.
 void dense_tile(pgx_program* P, int nlines, int rows) {
   const int64_t most = (smem_optin_max() - 4096) / (16 * (int64_t)P->lcap);  // slot and spare
-  if (nlines < 3 * 152 || most < 8) return;
+  if ((nlines < 3 * 152 && (int64_t)P->lcap * (((int64_t)nlines + 151) / 152) < 208) || most < 8) return;
   P->ops[1].k = (int16_t)(P->ops[1].k | PGX_DENSE_TC);
   P->tb = 8;
   const int rt = (rows + 15) / 16;
@@ -877,10 +878,11 @@ static bool composed_args(const double* in, const double* out, int nlines, int a
   return in && out && nlines >= 0 && axis >= 0 && axis <= 1;
 }
 
-// Where the transform is a long dense contraction of many lines, its rows are split over CTAs (dense_tile), which
-// the ops beside it cannot be: two passes (460 lines of 132 points, forward: 24 us against 31 as one).
+// Where the transform is a dense contraction on the FP16 tensor cores, its rows are split over CTAs (dense_tile),
+// which the ops beside it cannot be: two passes (460 lines of 132 points, forward: 24 us against 31 as one).
 extern "C" int pgx_stencil_one_pass(int32_t n, int32_t nlines) {
-  return nlines < 3 * 152 || n <= DENSE_MMA_MAX_N || pgx_fft_length_ok(n);
+  return n <= DENSE_MMA_MAX_N || pgx_fft_length_ok(n) ||
+         (nlines < 3 * 152 && ((int64_t)n + 2) * (((int64_t)nlines + 151) / 152) < 208);
 }
 
 extern "C" int pgx_stencil_values(const pgx_stencil_plan* p, const double* in, int64_t in_s0, int64_t in_s1, double* out,

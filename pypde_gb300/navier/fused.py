@@ -918,24 +918,80 @@ def _fft_slots(prog, sd=False):
 
 
 # A multi-slot DCT op saves barriers, but its FFT buffers take shared memory from the
-# tile: past this transform length each slot's lines alone fill the CTA's threads.
+# tile: in launches of many waves, past this transform length each slot's lines alone fill the CTA's threads.
 JOINT_DCT_MAX_N = 257
+SMS = 152
+
+
+def _pick_fft(prog, lines_total, lcap, fft_n):
+    """(lines per CTA, threads, one DCT op per slot) of a pass with FFTs whose CTAs are all resident at once or
+    make three waves at most; None for larger launches.
+
+    The stages of a transform end at barriers, so an SM is filled by CTAs that wait at different ones: the
+    smallest tile with three warps or more a CTA (the FFT build holds 768 threads an SM).  The DCTs of several
+    slots stay one op (fewer barriers) unless its FFT buffers keep CTAs off the SM that would otherwise be there,
+    up to four: P1 of 1149 lines of 433 points 36 us as one op and 42 slot by slot, of 577 points (room for three
+    of four CTAs) 58 and 49.  Against tiles of at least two CTAs an SM and slot-by-slot transforms from 289 points
+    on, as in launches of many waves: P2u of 769 lines of 385 points 34.2 -> 27.0 us, P2 of 2307 such lines
+    111 -> 88 (two waves), of 1299 lines of 577 points 150 -> 119."""
+    def room(tb, sd):
+        fs = _fft_slots(prog, sd)
+        # a CTA: the slots and FFT buffers, its descriptor, 1 KB of the system's
+        return (SMEM_PER_SM + 1024) // (tb * (8 * (prog.nslots + 1) * lcap + fs * fft_bytes_per_line(fft_n, fs == 1))
+                                        + ctypes.sizeof(_lib.PgxInstance) + 1040)
+
+    def per_sm(tb):
+        return max(1, -(-(-(-lines_total // tb)) // SMS))
+
+    sd = _fft_slots(prog) > 1 and room(2, False) < min(per_sm(2), 4)
+    for tb in range(2, 17, 2):
+        k = per_sm(tb)
+        nt = _lib.MAX_THREADS_FFT // k // 32 * 32
+        if k <= room(tb, sd) and nt >= 96:
+            return tb, min(nt, 384 if fft_n > 500 and k <= 2 else 256), sd
+        fit = min(room(2, sd), 4)
+        if tb == 2 and fit > 0 and k <= 3 * fit:
+            return 2, min(256, _lib.MAX_THREADS_FFT // fit // 32 * 32), sd
+    return None
+
+
+def _pick_warp_chains(lines_total, width, tbmax):
+    """Lines per CTA and threads of a pass whose chains run a warp each (``width`` a line): one line a CTA while
+    every CTA can be resident with four warps or more (1024 threads an SM), and warps for all its chains at once
+    or for equal rounds of them.  The ADI x-sweep of 385 lines of 289 points (12 chains a line): 54 us in CTAs of
+    one line and 192 threads, 58 in 128, 93 in CTAs of two lines and a warp for each of their 24 chains."""
+    tb = 1
+    while True:
+        per_sm = -(-(-(-lines_total // tb)) // SMS)
+        avail = _lib.MAX_THREADS // max(per_sm, 1) // 32 * 32
+        if avail >= 128 or 2 * tb > tbmax:
+            break
+        tb *= 2
+    avail = max(avail, 128)
+    chains = width * tb
+    rounds = -(-32 * chains // avail)
+    nt = 32 * -(-chains // rounds)
+    return tb, max(nt, min(256, avail)) if rounds == 1 else nt
 
 
 def _pick(prog, lines_total, lcap, fft_n, max_lines):
     """Lines per CTA and threads for one pass over ``lines_total`` lines (all instances).
 
-    FFT passes: at most ~113 KB of shared memory per CTA so two CTAs share an SM
+    FFT passes of many waves: at most ~113 KB of shared memory per CTA so two CTAs share an SM
     (one computes while the other waits at a barrier).  Passes dominated by
     sequential banded sweeps: many lines per CTA, because each (line, parity)
     chain is one thread and the FP64 pipe of every SM sub-partition needs a
     warp of chains.
     """
     nbuf = prog.nslots + 1
+    chains = any(o.code in [_lib.OP[k] for k in CHAIN_OPS] for o in prog.ops)
+    if fft_n > 1 and not chains and prog.has_dct:
+        few = _pick_fft(prog, lines_total, lcap, fft_n)
+        if few:
+            return few[0], few[1], False, few[2], False
     sd = _fft_slots(prog) > 1 and fft_n > JOINT_DCT_MAX_N
     fs = _fft_slots(prog, sd)
     per_line = 8 * nbuf * lcap + fs * fft_bytes_per_line(fft_n, fs == 1)
-    chains = any(o.code in [_lib.OP[k] for k in CHAIN_OPS] for o in prog.ops)
     if fft_n > 1:
         budget = SMEM_PER_SM // 2 - 2048
         cap = 16
@@ -946,16 +1002,16 @@ def _pick(prog, lines_total, lcap, fft_n, max_lines):
         budget = SMEM_PER_SM // 2 - 2048
         cap = 32
     tbmax = max(1, budget // per_line)
-    want = max(1, -(-lines_total // (2 * 152)))  # at least two CTAs per SM when there is work
+    want = max(1, -(-lines_total // (2 * SMS)))  # at least two CTAs per SM when there is work
     tb = max(1, min(cap, tbmax, want, max(max_lines, 1)))
     if fft_n > 1:
         tb = min(max(tb, 2), max(2, tbmax - tbmax % 2))
         tb -= tb % 2
-    elif _dense_tc(prog, lines_total, 256, fft_n, False):
+    elif _dense_tc(prog, lines_total, lcap, 256, fft_n, False):
         # eight lines an instruction, there or not: eight a CTA where the launch splits the rows over CTAs
         # (LOAD, DENSE, STORE), else as many as still leave every SM a CTA
         tb = 8 if len(prog.ops) == 3 else 1
-        while tb < 8 and -(-lines_total // tb) > 152:
+        while tb < 8 and -(-lines_total // tb) > SMS:
             tb *= 2
         tb = min(tb, tbmax)
     # one thread per (slot, line, parity) chain of the widest chain op
@@ -967,23 +1023,35 @@ def _pick(prog, lines_total, lcap, fft_n, max_lines):
             width = max(width, max(o.b, 1))
     nt = max(256, 32 * -(-width * tb // 32))
     # few chains in the whole launch: one warp per chain (scanned) instead of one thread
-    wc = chains and width * lines_total < 152 * 64
+    wc = chains and width * lines_total < SMS * 64
     ntmax = _max_threads(prog, fft_n, False)
-    if wc:
+    if wc and fft_n <= 1:
+        tb, nt = _pick_warp_chains(lines_total, width, min(tbmax, max(max_lines, 1)))
+    elif wc:
         nt = max(256, min(ntmax, 32 * width * tb))
     return tb, min(nt, ntmax), bool(wc), sd, False
 
 
-# Dense operators go to the tensor cores in digits (PGX_DENSE_TC) in launches of at least this many lines and CTAs
-# of at most that many threads.  An instruction takes eight lines, so a launch needs a few lines an SM to fill
-# them: 511 lines of 257 points 31 us against 72 as FP64 chains, 127 lines of 129 points 11 against 8.
-DENSE_TC_LINES = 3 * 152
+# Dense operators go to the tensor cores in digits (PGX_DENSE_TC) in launches of at least DENSE_TC_LINES lines and
+# CTAs of at most MAX_THREADS_DENSE threads.  An instruction takes eight lines, so a launch needs a few lines an SM
+# to fill them.  Where nothing but a load and a store goes with the operator the launch splits its rows over CTAs,
+# and the FP64 form, one wave of rows x columns a CTA after the other, loses from about 200 rows x waves on,
+# however few the lines (DENSE_TC_ROWS): 8 lines of 257 points 20 us against 35, 129 lines of 129 points 13.8
+# against 11.1, 193 such lines 13.6 against 15.3, 383 lines of 385 points 33 against 115.  With other ops beside
+# it: 383 lines of 193 points 34 against 38, 255 of 257 points 44 against 42, 511 of 257 points 46 against 75.
+DENSE_TC_LINES = 3 * SMS
+DENSE_TC_ROWS = 208
 MAX_THREADS_DENSE = 256
 
 
-def _dense_tc(prog, lines_total, nt, fft_n, dm):
-    return (lines_total >= DENSE_TC_LINES and nt <= MAX_THREADS_DENSE and (fft_n <= 1 or dm or not prog.has_dct)
-            and (dm or any(o.code == _lib.OP["DENSE"] for o in prog.ops)))
+def _dense_tc(prog, lines_total, lcap, nt, fft_n, dm):
+    if nt > MAX_THREADS_DENSE or (fft_n > 1 and not dm and prog.has_dct):
+        return False
+    if not (dm or any(o.code == _lib.OP["DENSE"] for o in prog.ops)):
+        return False
+    if len(prog.ops) == 3 and lcap * -(-lines_total // SMS) >= DENSE_TC_ROWS:
+        return True
+    return lines_total >= DENSE_TC_LINES or (4 * lines_total >= 3 * DENSE_TC_LINES and lcap >= 192)
 
 
 def _max_threads(prog, fft_n, dm):
@@ -1187,7 +1255,7 @@ class FusedBatch:
         DENSE op on the FP64 tensor cores (no FFT buffers)."""
         nv = len(prog.variants)
         lines_total = sum(self.insts[k].lines(prog) for k in members) * nv
-        P = launch_program(prog, key, tb, nt, wc, sd, dm, _dense_tc(prog, lines_total, nt, key[1], dm))
+        P = launch_program(prog, key, tb, nt, wc, sd, dm, _dense_tc(prog, lines_total, key[0], nt, key[1], dm))
         # the batched launch cannot read its descriptors on the host: check every member's host copy
         host = getattr(d_insts, "pgx_host", None)
         if host is None:
