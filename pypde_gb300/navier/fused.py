@@ -1249,13 +1249,16 @@ class FusedBatch:
         d.pgx_host = insts
         return d
 
-    def _group_launch(self, prog, d_insts, key, members, tb, nt, wc=False, name=None, sd=False, dm=False):
+    def _group_launch(self, prog, d_insts, key, members, tb, nt, wc=False, name=None, sd=False, dm=False, tc=None):
         """One launch of ``prog`` over ``members``; ``wc``: chain ops in warp-per-chain mode;
         ``sd``: multi-slot DCT ops as one op per slot; ``dm``: DCT ops as dense matrices and every
-        DENSE op on the FP64 tensor cores (no FFT buffers)."""
+        DENSE op on the FP64 tensor cores (no FFT buffers); ``tc``: DENSE ops in digits, by default
+        where ``_dense_tc`` has it."""
         nv = len(prog.variants)
         lines_total = sum(self.insts[k].lines(prog) for k in members) * nv
-        P = launch_program(prog, key, tb, nt, wc, sd, dm, _dense_tc(prog, lines_total, key[0], nt, key[1], dm))
+        if tc is None:
+            tc = _dense_tc(prog, lines_total, key[0], nt, key[1], dm)
+        P = launch_program(prog, key, tb, nt, wc, sd, dm, tc)
         # the batched launch cannot read its descriptors on the host: check every member's host copy
         host = getattr(d_insts, "pgx_host", None)
         if host is None:
@@ -1270,7 +1273,8 @@ class FusedBatch:
                 for t in range(-(-self.insts[k].lines(prog) // tb))]
         d_work = torch.as_tensor(np.asarray(work, dtype=np.int32).ravel(), device=device())
         return {"name": name or prog.name, "P": P, "d_insts": d_insts, "d_work": d_work, "nwork": len(work),
-                "key": key, "members": members, "prog": prog, "wc": bool(wc), "sd": bool(sd), "dm": bool(dm)}
+                "key": key, "members": members, "prog": prog, "wc": bool(wc), "sd": bool(sd), "dm": bool(dm),
+                "tc": bool(tc)}
 
     def _pass_launches(self, prog, tiles=None, stage=0, key_tiles=None):
         d_insts = self._d_insts(prog, stage)
@@ -1279,13 +1283,14 @@ class FusedBatch:
         for gi, (key, members) in enumerate(self._groups(prog)):
             lines = [self.insts[k].lines(prog) for k in members]
             tag = "%s#%d" % (name, gi)
+            tc = None
             if key_tiles and (name, key) in key_tiles:
-                tb, nt, wc, sd, dm = key_tiles[(name, key)]
+                tb, nt, wc, sd, dm, tc = key_tiles[(name, key)]
             elif tiles and tag in tiles:
                 tb, nt, wc, sd, dm = (tuple(tiles[tag][:5]) + (False,) * 3)[:5]
             else:
                 tb, nt, wc, sd, dm = _pick(prog, sum(lines) * len(prog.variants), key[0], key[1], max(lines))
-            out.append(self._group_launch(prog, d_insts, key, members, tb, nt, bool(wc), name, bool(sd), bool(dm)))
+            out.append(self._group_launch(prog, d_insts, key, members, tb, nt, bool(wc), name, bool(sd), bool(dm), tc))
         return out
 
     def _build_launches(self, tiles=None):
@@ -1505,8 +1510,10 @@ class FusedBatch:
     # ------------------------------------------------- host-resident state
     def _subset(self, idx):
         """Launch set of the instances ``idx`` (same state, scratch and tables), each launch with
-        the tile this batch uses for the same pass and size class."""
-        key_tiles = {(L["name"], L["key"]): (L["P"].tb, L["P"].nthreads, L["wc"], L["sd"], L["dm"])
+        the tile this batch uses for the same pass and size class, and its form of the dense ops: a tile
+        tuned for the digit products is no tile for FP64 chains, whichever form so few lines would take
+        by themselves (eight flows of up to 113 points a side: 1770 us a step against 940)."""
+        key_tiles = {(L["name"], L["key"]): (L["P"].tb, L["P"].nthreads, L["wc"], L["sd"], L["dm"], L["tc"])
                      for group in self.launches for L in group}
         sub = FusedBatch.__new__(FusedBatch)
         sub.solvers, sub.insts = [self.solvers[i] for i in idx], [self.insts[i] for i in idx]
