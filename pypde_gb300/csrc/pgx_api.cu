@@ -345,7 +345,7 @@ int twiddles(int n, const double** out) {
     return PGX_OK;
   }
   // L complex twiddles, then the fold coefficients 1/2 - sin(pi m / N) (m < N = L/2), each the
-  // FP64 sum 0.5 + Im(tw[m]) that the kernels would otherwise form per point
+  // FP64 sum 0.5 + Im(tw[m]) (the layout that callers know; the transform reads the entries after them)
   const int N = L / 2;
   const bool even = (N & 1) == 0;  // the folded transform also reads fixed-point twiddles
   std::vector<double> h(2 * (size_t)L + N + (even ? 2 * ((size_t)L + 1) : 0));
@@ -527,12 +527,14 @@ void pick_tile(pgx_program* P, int nlines, int maxlen, int nbuf, int fft_n) {
 
 // A LOAD, DENSE, STORE pass on the tensor cores, where that pays: an instruction takes eight lines whether they
 // are there or not, and the launch splits the rows over CTAs; the FP64 chains take one wave of lines after the
-// other, rows x columns each.  They lose from about 200 rows x waves on: 8 lines of 257 points 20 us against 35,
+// other, rows x columns each.  They lose from about 200 x 200 in one wave on: 8 lines of 257 points 20 us against 35,
 // 129 lines of 129 points 13.8 against 11.1, 193 such lines 13.6 against 15.3, 400 lines of 385 points 39 against
 // 128.  Eight lines a CTA, a warp per row block up to eight.
-void dense_tile(pgx_program* P, int nlines, int rows) {
+void dense_tile(pgx_program* P, int nlines, int rows, int cols) {
   const int64_t most = (smem_optin_max() - 4096) / (16 * (int64_t)P->lcap);  // slot and spare
-  if ((nlines < 3 * 152 && (int64_t)P->lcap * (((int64_t)nlines + 151) / 152) < 208) || most < 8) return;
+  const int64_t waves = ((int64_t)nlines + 151) / 152;
+  if (rows < 32 || cols < 32 || most < 8) return;  // thin operators (two-mode boundary bases) are a few products a row
+  if (nlines < 3 * 152 && (int64_t)rows * cols * waves * waves < 208 * 208) return;
   P->ops[1].k = (int16_t)(P->ops[1].k | PGX_DENSE_TC);
   P->tb = 8;
   const int rt = (rows + 15) / 16;
@@ -597,7 +599,7 @@ int pgx_dct_pass(const double* in, int64_t in_s0, int64_t in_s1, int32_t n_in, d
   }
   P.ops[2] = mk(PGX_OP_STORE, 0, -1, 1);
   pick_tile(&P, nlines, n, 2, P.fft_n);
-  if (!fft && !mma) dense_tile(&P, nlines, n);
+  if (!fft && !mma) dense_tile(&P, nlines, n, n);
   if (mma) {  // one 8-line tensor-core tile per CTA, a warp per 8-row block
     P.tb = 8;
     P.nthreads = 32 * ((n + 7) / 8);
@@ -882,7 +884,7 @@ static bool composed_args(const double* in, const double* out, int nlines, int a
 // which the ops beside it cannot be: two passes (460 lines of 132 points, forward: 24 us against 31 as one).
 extern "C" int pgx_stencil_one_pass(int32_t n, int32_t nlines) {
   return n <= DENSE_MMA_MAX_N || pgx_fft_length_ok(n) ||
-         (nlines < 3 * 152 && ((int64_t)n + 2) * (((int64_t)nlines + 151) / 152) < 208);
+         (nlines < 3 * 152 && (int64_t)n * (((int64_t)nlines + 151) / 152) < 208);
 }
 
 extern "C" int pgx_stencil_values(const pgx_stencil_plan* p, const double* in, int64_t in_s0, int64_t in_s1, double* out,
@@ -1282,6 +1284,6 @@ extern "C" int pgx_matrix_apply(const pgx_matrix_plan* p, const double* in, int6
   }
   P.ops[2] = mk(PGX_OP_STORE, 0, -1, 1);
   pick_tile(&P, nlines, p->rows > p->cols ? p->rows : p->cols, 2, 0);
-  if (!p->banded) dense_tile(&P, nlines, p->rows);
+  if (!p->banded) dense_tile(&P, nlines, p->rows, p->cols);
   return pgx_run(&P, &I, stream);
 }
